@@ -172,7 +172,8 @@ __global__ void __launch_bounds__(kThreads) extract_kernel(const __grid_constant
     }
 }
 
-__global__ void __launch_bounds__(kThreads) transform_kernel(unsigned char* points, int64_t n, Pose P) {
+// Clouds that do not start on 16 bytes: a point's position moved byte by byte.
+__global__ void __launch_bounds__(kThreads) transform_bytes_kernel(unsigned char* points, int64_t n, Pose P) {
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     unsigned char* pt = points + i * kPointBytes;
@@ -181,6 +182,55 @@ __global__ void __launch_bounds__(kThreads) transform_kernel(unsigned char* poin
     float w[3];
     apply_pose(P, v[0], v[1], v[2], w);
     memcpy(pt, w, 12);
+}
+
+// A CTA takes kThreads points, 33 x 256 bytes that start on 16, into shared
+// memory as 16-byte vectors, changes the positions there and writes the tile
+// back whole: every sector of a cloud holds part of a position, so its bytes
+// bound the kernel, read once and written once.  In shared memory a position
+// covers three or four words; a word it shares belongs otherwise to the same
+// point's later bytes or to the point before, neither of which is written, so
+// no two threads write one word.  (Word 33 i / 4 of lane i: no bank conflicts.)
+// 2.46 M points: about 37 us (162 MB moved), 154 us with a byte load and a byte
+// store for each of a position's 12 bytes.
+__global__ void __launch_bounds__(kThreads) transform_kernel(unsigned char* points, int64_t n, Pose P) {
+    constexpr int kTileBytes = kThreads * kPointBytes;
+    static_assert(kTileBytes % 16 == 0, "tiles start on 16 bytes");
+    __shared__ __align__(16) uint32_t s_tile[kTileBytes / 4];
+    const int64_t first = (int64_t)blockIdx.x * kThreads;
+    unsigned char* tile = points + first * kPointBytes;
+    const int bytes = (int)((n - first < kThreads ? n - first : kThreads) * kPointBytes);
+    const int vecs = bytes / 16;
+    unsigned char* sb = reinterpret_cast<unsigned char*>(s_tile);
+    for (int k = threadIdx.x; k < vecs; k += kThreads)
+        reinterpret_cast<uint4*>(s_tile)[k] = reinterpret_cast<const uint4*>(tile)[k];
+    if ((int)threadIdx.x < bytes - 16 * vecs) sb[16 * vecs + threadIdx.x] = tile[16 * vecs + threadIdx.x];
+    __syncthreads();
+    if (first + threadIdx.x < n) {
+        const int at = (int)threadIdx.x * kPointBytes;
+        uint32_t* w = s_tile + (at >> 2);
+        const unsigned sh = 8u * (unsigned)(at & 3);
+        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = sh ? w[3] : 0u;
+        float c[3];
+        apply_pose(P, __uint_as_float(__funnelshift_r(w0, w1, sh)), __uint_as_float(__funnelshift_r(w1, w2, sh)),
+                   __uint_as_float(__funnelshift_r(w2, w3, sh)), c);
+        const uint32_t x = __float_as_uint(c[0]), y = __float_as_uint(c[1]), z = __float_as_uint(c[2]);
+        if (sh) {
+            const uint32_t low = (1u << sh) - 1u;   // the bytes of word 0 below the position, of word 3 in it
+            w[0] = (w0 & low) | (x << sh);
+            w[1] = __funnelshift_l(x, y, sh);
+            w[2] = __funnelshift_l(y, z, sh);
+            w[3] = (z >> (32u - sh)) | (w3 & ~low);
+        } else {
+            w[0] = x;
+            w[1] = y;
+            w[2] = z;
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < vecs; k += kThreads)
+        reinterpret_cast<uint4*>(tile)[k] = reinterpret_cast<const uint4*>(s_tile)[k];
+    if ((int)threadIdx.x < bytes - 16 * vecs) tile[16 * vecs + threadIdx.x] = sb[16 * vecs + threadIdx.x];
 }
 
 // The position of point i: its 12 bytes start at byte i & 3 of a word when the
@@ -361,8 +411,12 @@ gbt_status gbt_points_transform(gbt_point* points, int64_t n, const double pose[
     if (n <= 0) return fail(GBT_ERR_INVALID_ARG, fn, "the number of points is 0");
     if (n > (int64_t)0xffffffffll) return fail(GBT_ERR_INVALID_ARG, fn, "point count above 2^32-1");
     cudaGetLastError();
-    transform_kernel<<<blocks_for(n), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<unsigned char*>(points), n, make_pose(pose));
+    unsigned char* bytes = reinterpret_cast<unsigned char*>(points);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if ((reinterpret_cast<uintptr_t>(points) & 15u) == 0)
+        transform_kernel<<<blocks_for(n), kThreads, 0, st>>>(bytes, n, make_pose(pose));
+    else
+        transform_bytes_kernel<<<blocks_for(n), kThreads, 0, st>>>(bytes, n, make_pose(pose));
     return cuda_status(fn);
 }
 

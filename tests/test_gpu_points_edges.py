@@ -49,3 +49,19 @@ def test_project_from_any_byte(gpu, engine_lib, oracle, offset, n):
     assert np.array_equal(depth.cpu().numpy().view(np.uint32), ed.view(np.uint32))
     assert np.array_equal(rgb.cpu().numpy(), ec)
     assert (ed > 0).any() or n < 31
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 8, 16])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 16, 255, 256, 257, 1000])
+def test_transform_from_any_byte(gpu, engine_lib, oracle, offset, n):
+    """Every byte of the records, and none outside them."""
+    pts = cloud(oracle, n, 7 * n + offset)
+    buf, dev = at_byte(gpu, pts, offset)
+    pose = np.concatenate([[0.5, -0.5, 0.5, 0.5], [0.3, -1.2, 2.0]])
+    engine_lib.check(engine_lib.lib().gbt_points_transform(C.c_void_p(dev.data_ptr()), n,
+                                                           C.byref((C.c_double * 7)(*pose)), None))
+    gpu.cuda.synchronize()
+    oracle.points_transform(pts, pose)
+    exp = np.full(pts.nbytes + 64, 0xAB, np.uint8)
+    exp[offset:offset + pts.nbytes] = pts.reshape(-1)
+    assert np.array_equal(buf.cpu().numpy(), exp)
