@@ -81,6 +81,10 @@ class Frame(C.Structure):
     ]
 
 
+Pose7 = C.c_double * 7
+Matrix9 = C.c_double * 9
+
+
 # gbt_frame as a numpy record, for filling many frame descriptors at once
 FRAME_DTYPE = None
 
@@ -175,6 +179,8 @@ class GbtError(RuntimeError):
 def lib():
     """Load the engine library (raises if it has not been built)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):

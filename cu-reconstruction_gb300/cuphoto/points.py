@@ -36,12 +36,13 @@ def _log(msg):
 
 
 def _k9(m):
-    a = (C.c_double * 9)(*[float(x) for x in m])
-    return a
+    return L.Matrix9(*[float(x) for x in m])
 
 
 def _pose7(p):
-    return (C.c_double * 7)(*[float(x) for x in p])
+    if type(p) is np.ndarray and p.dtype == np.float64 and p.ndim == 1:
+        return L.Pose7(*p.tolist())
+    return L.Pose7(*[float(x) for x in p])
 
 
 class PointCloud:
@@ -106,21 +107,21 @@ class PointCloud:
             _log("cudaPointCloud::extract_points() -- depth width/height parameters are zero")
             return False
         L.device_image(depth, "depth", (torch.float32, torch.uint16, torch.int16))
-        H, W = int(depth.shape[0]), int(depth.shape[1])
-        fmt = L.DEPTH_U16 if depth.dtype in (torch.uint16, torch.int16) else L.DEPTH_F32_M
+        H, W = depth.shape
+        f32 = depth.dtype == torch.float32
         cptr, cpitch = None, 0
         if colors is not None:
             L.device_image(colors, "colors", (torch.uint8,), channels=3)
-            if tuple(colors.shape[:2]) != (H, W):
-                raise ValueError("colors are %dx%d, depth %dx%d" % (colors.shape[1], colors.shape[0], W, H))
+            cH, cW, _ = colors.shape
+            if (cH, cW) != (H, W):
+                raise ValueError("colors are %dx%d, depth %dx%d" % (cW, cH, W, H))
             self.has_rgb = True
-            cptr, cpitch = C.c_void_p(colors.data_ptr()), int(colors.stride(0) * colors.element_size())
+            cptr, cpitch = colors.data_ptr(), colors.stride(0)
         start = int(frame_idx) * W * H
-        st = L.lib().gbt_points_extract(C.byref(_k9(self.camera_matrix)), C.c_void_p(depth.data_ptr()),
-                                        int(depth.stride(0) * depth.element_size()), fmt, float(depth_scale), cptr,
-                                        cpitch, W, H, C.byref(_pose7(transform)), start,
-                                        C.c_void_p(self.device_pts.data_ptr()), self.total_num_pts,
-                                        _stream_handle(stream))
+        st = L.lib().gbt_points_extract(C.byref(_k9(self.camera_matrix)), depth.data_ptr(),
+                                        depth.stride(0) * (4 if f32 else 2), L.DEPTH_F32_M if f32 else L.DEPTH_U16,
+                                        float(depth_scale), cptr, cpitch, W, H, C.byref(_pose7(transform)), start,
+                                        self.device_pts.data_ptr(), self.total_num_pts, _stream_handle(stream))
         if st != L.GBT_OK:
             _log("cudaPointCloud::extract_points() -- " + L.lib().gbt_last_error().decode())
             return False
