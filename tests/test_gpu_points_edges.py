@@ -65,3 +65,62 @@ def test_transform_from_any_byte(gpu, engine_lib, oracle, offset, n):
     exp = np.full(pts.nbytes + 64, 0xAB, np.uint8)
     exp[offset:offset + pts.nbytes] = pts.reshape(-1)
     assert np.array_equal(buf.cpu().numpy(), exp)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4, 16])
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 1), (33, 3), (64, 8), (257, 5)])
+@pytest.mark.parametrize("fx,cx", [(525.0, 319.5), (-313.7, 30.0 + 1e-9), (1.0 / 3, 16.0 - 2.0 ** -30), (2.0 ** 21, 7.25),
+                                   (2.0 ** -21, 0.0)])
+def test_extract_any_start_and_camera(gpu, engine_lib, oracle, offset, w, h, fx, cx):
+    """Spans that do and do not start on 16 bytes, runs with and without depth,
+    centres next to a pixel, focal lengths on both sides of the limits of the
+    form without FP64, depths far outside a sensor's range."""
+    rng = np.random.default_rng(w * 1000 + h)
+    d = (rng.integers(1, 9000, (h, w)) * np.float32(0.001)).astype(np.float32)
+    odd = np.array([1e-12, 3e-9, 2.0 ** -30, 2e9, 1e30, np.inf, 1.5, 0.75, 1e-38, np.nan], np.float32)
+    d = np.where(rng.random((h, w)) < 0.2, odd[rng.integers(0, len(odd), (h, w))], d)
+    d[rng.random((h, w)) < (0.5 if h == 3 else 0.1)] = 0
+    rgb = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+    pose = np.concatenate([[0.5, -0.5, 0.5, 0.5], [0.3, -1.2, 2.0]])
+    K = np.array([fx, 0, 0, 0, 1.5 * fx, 0, cx, 0.5 * cx, 1.0])
+    start, n = 3, w * h + 5
+    exp = cloud(oracle, n, 11)
+    buf, dev = at_byte(gpu, exp, offset)
+    d_t, rgb_t = gpu.from_numpy(d).cuda(), gpu.from_numpy(rgb).cuda()
+    engine_lib.check(engine_lib.lib().gbt_points_extract(
+        C.byref((C.c_double * 9)(*K)), C.c_void_p(d_t.data_ptr()), 4 * w, engine_lib.DEPTH_F32_M, 1.0,
+        C.c_void_p(rgb_t.data_ptr()), 3 * w, w, h, C.byref((C.c_double * 7)(*pose)), start,
+        C.c_void_p(dev.data_ptr()), n, None))
+    gpu.cuda.synchronize()
+    got = buf.cpu().numpy()
+    assert (got[:offset] == 0xAB).all() and (got[offset + exp.nbytes:] == 0xAB).all()
+    oracle.points_extract(K, d, rgb, pose, exp, start=start)
+    a, b = (r.reshape(-1).copy().view(oracle.POINT_DTYPE) for r in (got[offset:offset + exp.nbytes], exp))
+    nan = np.isnan(a["pos"]) & np.isnan(b["pos"])   # (the payload of a NaN is the processor's)
+    a["pos"][nan] = b["pos"][nan] = 0
+    assert a.tobytes() == b.tobytes()
+
+
+def test_extract_runs_from_a_vector_boundary(gpu, engine_lib, oracle):
+    """The 16-byte form over every mix of pixels with and without depth in a span."""
+    w, h = 32, 512
+    rng = np.random.default_rng(5)
+    d = (rng.integers(1, 9000, (h, w)) * np.float32(0.001)).astype(np.float32)
+    for r in range(h):
+        if r % 4 == 1:
+            d[r, rng.random(w) < rng.random()] = 0
+        elif r % 4 == 2:
+            d[r, : r % 33] = 0
+        elif r % 4 == 3:
+            d[r, r % 33:] = 0
+    pose = np.concatenate([[0.5, -0.5, 0.5, 0.5], [0.3, -1.2, 2.0]])
+    K = np.array([525.0, 0, 0, 0, 525.0, 0, 319.5, 239.5, 1.0])
+    exp = cloud(oracle, w * h, 12)
+    buf, dev = at_byte(gpu, exp, 0)
+    d_t = gpu.from_numpy(d).cuda()
+    engine_lib.check(engine_lib.lib().gbt_points_extract(
+        C.byref((C.c_double * 9)(*K)), C.c_void_p(d_t.data_ptr()), 4 * w, engine_lib.DEPTH_F32_M, 1.0, None, 0, w, h,
+        C.byref((C.c_double * 7)(*pose)), 0, C.c_void_p(dev.data_ptr()), w * h, None))
+    gpu.cuda.synchronize()
+    oracle.points_extract(K, d, None, pose, exp)
+    assert np.array_equal(buf.cpu().numpy()[:exp.nbytes], exp.reshape(-1))
