@@ -90,8 +90,8 @@ struct gbt_volume {
     bool managed;
     void* tvox;
     // marching-cubes scratch: [0,64) header (ticket u32, error i32, total i64, tiles listed u32),
-    // then two u64 totals per superblock of 1024 tiles, one u64 word per tile, one bit per group
-    // of 32 cubes, and the u32 list of tiles with triangles
+    // then two u64 totals per superblock of 1024 tiles, four u64 of counts per tile, a bit per cube,
+    // the u32 list of tiles with triangles, a u64 offset per tile and the voxels' bit planes
     void* mc_scratch;
     size_t mc_scratch_bytes;
     // shared-vertex mesh scratch: used-edge bits, word offsets, block sums, vertex count
@@ -681,8 +681,17 @@ gbt_status mc_prepare(gbt_volume* v, float* verts, int32_t* tris, int64_t cap, i
     a->cap = cap;
     a->index_base = index_base;
     const size_t nsuper = (size_t)gbt::mc_superblocks(a->ntiles);
-    const size_t nwords = (size_t)gbt::mc_group_words(ncubes);
-    const size_t need = 64 + nsuper * 16 + (size_t)a->ntiles * 12 + nwords * 4;
+    const size_t nwords = (size_t)(ncubes + 31) / 32;
+    // the voxels that cubes read: all of them, in the compat mode those up to
+    // the last one of its layers gx + gy apart (marching_cubes.cu:211)
+    const bool fixed = v->cfg.mode == GBT_MODE_FIXED;
+    if (ncubes > 0)
+        a->nbits = fixed ? (uint32_t)v->nvox
+                         : (uint32_t)((int64_t)(d.nz - 1) * (d.nx + d.ny) + (int64_t)d.nx * d.ny);
+    const size_t plane = gbt::mc_bit_plane_bytes(a->nbits);
+    // totals, counts (32 B a tile), cube bits, offsets (8), list (64)
+    const size_t front = (64 + nsuper * 16 + (size_t)a->ntiles * 104 + nwords * 4 + 63) / 64 * 64;
+    const size_t need = front + (fixed ? 2 : 1) * plane;
     if (v->mc_scratch_bytes < need) {
         if (v->mc_scratch) cudaFree(v->mc_scratch);
         v->mc_scratch = nullptr;
@@ -700,18 +709,21 @@ gbt_status mc_prepare(gbt_volume* v, float* verts, int32_t* tris, int64_t cap, i
     a->total = reinterpret_cast<long long*>(s + 8);
     a->nonempty = reinterpret_cast<unsigned int*>(s + 16);
     a->super = reinterpret_cast<unsigned long long*>(s + 64);
-    a->status = a->super + 2 * nsuper;
-    a->group_bits = reinterpret_cast<uint32_t*>(a->status + a->ntiles);
-    a->tile_list = a->group_bits + nwords;
+    a->counts = a->super + 2 * nsuper;
+    a->cube_bits = reinterpret_cast<uint32_t*>(a->counts + 4 * (size_t)a->ntiles);
+    a->status = reinterpret_cast<unsigned long long*>(s + front - (size_t)a->ntiles * 8);
+    a->tile_list = a->cube_bits + nwords;
+    a->bits_s = reinterpret_cast<uint32_t*>(s + front);
+    a->bits_o = fixed ? reinterpret_cast<uint32_t*>(s + front + plane) : nullptr;
     return GBT_OK;
 }
 
 gbt_status mc_launch(gbt_volume* v, const gbt::McArgs& a, cudaStream_t s) {
     cudaGetLastError();  // a launch reports only its own failure
-    // header, superblock totals, tile words and group bits start at zero
+    // header, superblock totals, tile words and cube bits start at zero
     cudaError_t e = cudaMemsetAsync(v->mc_scratch, 0,
-                                    64 + (size_t)gbt::mc_superblocks(a.ntiles) * 16 + (size_t)a.ntiles * 8 +
-                                        (size_t)gbt::mc_group_words(a.ncubes) * 4, s);
+                                    64 + (size_t)gbt::mc_superblocks(a.ntiles) * 16 + (size_t)a.ntiles * 32 +
+                                        ((size_t)a.ncubes + 31) / 32 * 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "mesh scratch clear");
     if (a.ntiles == 0) return GBT_OK;
     if (v->cfg.mode == GBT_MODE_FIXED)

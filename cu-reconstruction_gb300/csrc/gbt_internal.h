@@ -152,6 +152,13 @@ constexpr int kMcTileMin = kMcThreads * 4;   // the smallest tile of either mode
 constexpr int kMcSuperShift = 10;               // tiles per superblock of the tile scan: 1024
 inline int64_t mc_superblocks(int64_t ntiles) { return (ntiles + (1 << kMcSuperShift) - 1) >> kMcSuperShift; }
 inline int64_t mc_group_words(int64_t ncubes) { return (ncubes + 1023) / 1024; }
+// Bit planes of the marching cubes (a voxel's bit at its linear number) in
+// chunks of 512 voxels, 16 words; a spare chunk of zeros ends them, so that
+// the word after a voxel's can always be read.
+__host__ __device__ inline uint32_t mc_bit_chunks(uint32_t nbits) {
+    return (uint32_t)(((uint64_t)nbits + 511) / 512 + 1);
+}
+inline size_t mc_bit_plane_bytes(uint32_t nbits) { return (size_t)mc_bit_chunks(nbits) * 64; }
 // Triangle t of a mesh without shared vertices has the int32 indices
 // index_base + 3t, +1, +2: a capacity whose last index would pass
 // INT32_MAX, or a negative base, is refused before anything is written
@@ -178,15 +185,22 @@ struct McArgs {
     int32_t* tris;
     int64_t cap;
     int64_t index_base;
-    unsigned long long* status;  // [ntiles] triangles per tile, then exclusive offsets; zeroed before launch
-    unsigned long long* super;   // [ceil(ntiles / 1024)][2] triangles and tiles with triangles per
+    unsigned long long* counts;  // row walks: [ntiles] triangles per tile; bit planes: [ntiles][4], 16 bits for
+                                 // each sixteenth of a tile; zeroed before launch
+    unsigned long long* status;  // [ntiles] exclusive offsets of the tiles' triangles (may be counts' words)
+    unsigned long long* super;   // [ceil(ntiles / 1024)][2] triangles and list entries per
                                  // superblock of 1024 tiles; zeroed before launch
-    uint32_t* tile_list;         // [ntiles] tiles with triangles, in order
-    uint32_t* group_bits;        // [ceil(ncubes / 1024)] bit g: group g of 32 cubes has triangles; zeroed
+    uint32_t* tile_list;         // tiles with triangles, in order; with bit planes up to 16 entries a tile
+    uint32_t* group_bits;        // row walks: [ceil(ncubes / 1024)] bit g: group g of 32 cubes has triangles; zeroed
+    uint32_t* cube_bits;         // bit planes: [ceil(ncubes / 32)] bit c: cube c has triangles; zeroed
     unsigned int* nonempty;      // length of tile_list
     unsigned int* ticket;        // emission ticket, zeroed before launch
     long long* total;            // triangle count out
     int* error;                  // stays 0: no launch waits on another CTA
+    uint32_t* bits_s;            // bit planes of the first nbits voxels, or NULL (counts by row walks):
+    uint32_t* bits_o;            // distance below zero; fixed mode: weight above zero
+    uint32_t nbits;
+    uint32_t pad1;
     // Fixed mode with shared vertices: when edge_bits is set, triangles are
     // written as indices of the vertices of their grid edges (edge
     // 3 * voxel + axis; vertex index = edge_word_offset[edge / 32] + the set

@@ -19,7 +19,9 @@
 #error "define GBT_ARITH_NS (one namespace per arithmetic translation unit)"
 #endif
 
-#define GBT_MC_CONST static __constant__
+// (global memory: the kernels copy them to shared memory with coalesced loads,
+// which the constant cache would serve one word at a time)
+#define GBT_MC_CONST static __device__ const
 #include "mc_tables.inc"
 GBT_MC_TABLE_DATA
 #undef GBT_MC_CONST
@@ -1172,91 +1174,6 @@ __device__ __forceinline__ bool cube_xcorners(const McArgs& a, uint32_t c, uint3
     return cx + 2 == gx;
 }
 
-// Types (0 for a cube that is not emitted: past the end, or in the fixed mode
-// with a corner of weight <= 0) of NG consecutive groups of 32 cubes from
-// cube `base` (a multiple of 32): lane l of group i holds cube
-// base + 32 i + l.  Every x-corner load of the NG groups is issued before any
-// is used.  The x + 1 corners of a cube are the next lane's x corners, or
-// for lane 31 the x corners of lane 0 of the next group; the last cube of a
-// grid row and lane 31 of the last group load theirs, under a branch the
-// warp takes only when one of its lanes needs it.  A cube past the end reads
-// the last cube, in bounds, and is discarded.
-template <int MODE, int NG>
-__device__ __forceinline__ void mc_warp_types(const McArgs& a, uint64_t base, int lane, int (&type)[NG],
-                                              const unsigned char* s_type) {
-    bool own[NG];
-    float dx[NG][4], wx[NG][4];
-#pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        const uint64_t cube = base + 32 * i + lane;
-        const uint32_t c = cube < a.ncubes ? (uint32_t)cube : a.ncubes - 1;
-        uint32_t idx[4];
-        own[i] = cube_xcorners<MODE>(a, c, idx) || (i == NG - 1 && lane == 31);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            dx[i][k] = __ldg(a.D + idx[k]);
-            if (MODE == kFixed) wx[i][k] = __ldg(a.W + idx[k]);
-        }
-    }
-    int so[NG];
-#pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        so[i] = 0;
-        if (__any_sync(0xffffffffu, own[i]) && own[i]) {
-            // (the corner indices again, rather than kept live for the rare case)
-            const uint64_t cube = base + 32 * i + lane;
-            uint32_t idx[4];
-            cube_xcorners<MODE>(a, cube < a.ncubes ? (uint32_t)cube : a.ncubes - 1, idx);
-            bool ok = true;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                so[i] |= (__ldg(a.D + idx[k] + 1) < 0.f) << k;
-                if (MODE == kFixed) ok = ok && __ldg(a.W + idx[k] + 1) > 0.f;
-            }
-            if (MODE == kFixed) so[i] |= ok << 4;
-        }
-    }
-    int sx[NG];
-#pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        sx[i] = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) sx[i] |= (dx[i][k] < 0.f) << k;
-        if (MODE == kFixed) {
-            const bool okx = wx[i][0] > 0.f && wx[i][1] > 0.f && wx[i][2] > 0.f && wx[i][3] > 0.f;
-            sx[i] |= okx << 4;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        // every lane takes part in both shuffles
-        const int nx = __shfl_down_sync(0xffffffffu, sx[i], 1);
-        const int nf = __shfl_sync(0xffffffffu, sx[i + 1 < NG ? i + 1 : i], 0);
-        const int sn = own[i] ? so[i] : (lane == 31 ? nf : nx);
-        const int t = s_type[(sx[i] & 15) | (sn & 15) << 4];
-        bool ok = base + 32 * i + lane < a.ncubes;
-        if (MODE == kFixed) ok = ok && (sx[i] & sn & 16);
-        type[i] = ok ? t : 0;
-    }
-}
-
-// Types of the thread's cubes of a tile: warp w holds the CPT consecutive
-// groups of 32 cubes from group w * CPT, classified NB groups at a time (the
-// fixed mode also loads weights: half as many in flight).
-template <int MODE, int CPT>
-__device__ __forceinline__ void mc_tile_types(const McArgs& a, uint32_t tile, int tid, int (&type)[CPT],
-                                              const unsigned char* s_type) {
-    constexpr int NB = MODE == kFixed ? 2 : 4;
-    const uint64_t base = (uint64_t)tile * (kMcThreads * CPT) + (uint64_t)(tid >> 5) * (32 * CPT);
-#pragma unroll
-    for (int i0 = 0; i0 < CPT; i0 += NB) {
-        int t[NB];
-        mc_warp_types<MODE, NB>(a, base + 32 * i0, tid & 31, t, s_type);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) type[i0 + i] = t[i];
-    }
-}
-
 __device__ __forceinline__ void mc_load_tables(unsigned char* s_count, unsigned long long* s_tri, unsigned char* s_ends,
                                                unsigned char* s_type) {
     for (int k = threadIdx.x; k < 256; k += blockDim.x) {
@@ -1267,7 +1184,11 @@ __device__ __forceinline__ void mc_load_tables(unsigned char* s_count, unsigned 
     if (s_ends && threadIdx.x < 12) s_ends[threadIdx.x] = GBT_MC_EDGE_ENDS[threadIdx.x];
 }
 
-// Marching cubes in four launches, none of which waits on another CTA.
+// Marching cubes in five launches, none of which waits on another CTA:
+// mc_bits_kernel and mc_bitcount_kernel (bit planes, counts), mc_reduce_kernel
+// and mc_scan_kernel (offsets), mc_emit_cubes_kernel.  In four where the
+// scratch has no room for bit planes (gbt_extract_mesh_noalloc), with (1) and
+// (3) instead:
 // (1) mc_count_kernel: a warp takes a segment of kMcSegCubes cubes along x in
 //     one cube layer and walks kMcRowsPerTask rows along y.  Lane l holds
 //     voxel column x0 + l; per row it loads its voxels at (y+1, z) and
@@ -1288,7 +1209,33 @@ __device__ __forceinline__ void mc_load_tables(unsigned char* s_count, unsigned 
 // from the words afterwards, by mc_reduce_kernel: atomics on them from the
 // rows of every warp contend for a few addresses.)
 __device__ __forceinline__ void mc_add_tile(const McArgs& a, uint64_t t, unsigned n) {
-    atomicAdd(a.status + t, (unsigned long long)n);
+    atomicAdd(a.counts + t, (unsigned long long)n);
+}
+// Counting from bit planes keeps 16 counts a tile, one for each of its
+// sixteenths (p), 16 bits each (at most 5 x 128 triangles) in four words.
+__device__ __forceinline__ void mc_add_part(const McArgs& a, uint64_t t, unsigned p, unsigned n) {
+    atomicAdd(a.counts + 4 * t + (p >> 2), (unsigned long long)n << (16u * (p & 3u)));
+}
+__device__ __forceinline__ unsigned mc_tile_triangles(const McArgs& a, uint64_t t) {
+    if (!a.bits_s) return (unsigned)a.counts[t];
+    unsigned n = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned long long c = a.counts[4 * t + k];
+        const unsigned long long pair = (c & 0x0000ffff0000ffffull) + (c >> 16 & 0x0000ffff0000ffffull);
+        n += (unsigned)pair + (unsigned)(pair >> 32);
+    }
+    return n;
+}
+// Entries of the list of tiles: one for a tile with few triangles, four
+// (quarters) or sixteen for more, so that no warp of the emission has much
+// more to do than another: a flat surface along x fills tiles with two
+// thousand triangles (with quarters as the smallest parts the emission took
+// 82 us instead of 70 at 512^3).  (The row walks' tiles are emitted whole.)
+constexpr unsigned kMcWholeTile = 96, kMcQuarterTile = 384;   // triangles up to which a tile is one entry, or four
+__device__ __forceinline__ unsigned mc_tile_entries(const McArgs& a, unsigned triangles) {
+    if (triangles == 0u) return 0u;
+    return !a.bits_s || triangles <= kMcWholeTile ? 1u : triangles <= kMcQuarterTile ? 4u : 16u;
 }
 
 constexpr uint32_t kMcSegCubes = 31;      // cubes per segment: 32 voxel columns
@@ -1590,18 +1537,170 @@ __global__ void __launch_bounds__(kMcThreads) mc_count4_kernel(const __grid_cons
     }
 }
 
+// Counting from bit planes, wherever the volume can keep them (1 bit per voxel,
+// 2 in the fixed mode; gbt_extract_mesh_noalloc's static scratch cannot, it
+// takes the row-walking kernels above).
+//
+// (1a) mc_bits_kernel streams the distances (and weights) once, as a copy
+// would, and keeps a voxel's sign (and whether it was observed) as a bit of its
+// linear number.  Bound by HBM: 1.07 GB at 512^3 in 170 us, 6.3 TB/s.  A warp
+// holds 16 words of 32 voxels of each grid in flight, one coalesced load and
+// one ballot a word.  With the count below, 197 us against 248 for the row
+// walk, which reads every voxel twice and is bound by the loads a warp keeps in
+// flight between its rows.
+constexpr uint32_t kMcBitVoxels = 512;   // voxels of a warp's step
+
+template <int MODE>
+__global__ void __launch_bounds__(kMcThreads) mc_bits_kernel(const __grid_constant__ McArgs a) {
+    constexpr int K = (int)kMcBitVoxels / 32;
+    const int lane = threadIdx.x & 31;
+    const uint32_t nchunks = mc_bit_chunks(a.nbits);
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < nchunks; chunk += nwarps) {
+        const uint64_t first = (uint64_t)chunk * kMcBitVoxels + (uint64_t)lane;
+        float d[K], w[MODE == kFixed ? K : 1];
+        if ((uint64_t)(chunk + 1) * kMcBitVoxels <= a.nbits) {   // the same for the whole warp
+#pragma unroll
+            for (int k = 0; k < K; ++k) d[k] = __ldg(a.D + first + 32 * k);
+            if (MODE == kFixed) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) w[k] = __ldg(a.W + first + 32 * k);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const bool in = first + 32 * k < a.nbits;
+                d[k] = in ? __ldg(a.D + first + 32 * k) : 0.f;
+                if (MODE == kFixed) w[k] = in ? __ldg(a.W + first + 32 * k) : 0.f;
+            }
+        }
+        uint32_t mine = 0u;   // lane k: sign word k; lane 16 + k: observed word k
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t s = __ballot_sync(0xffffffffu, d[k] < 0.f);
+            if (lane == k) mine = s;
+            if (MODE == kFixed) {
+                const uint32_t o = __ballot_sync(0xffffffffu, w[k] > 0.f);
+                if (lane == K + k) mine = o;
+            }
+        }
+        if (lane < K)
+            a.bits_s[chunk * K + lane] = mine;
+        else if (MODE == kFixed)
+            a.bits_o[chunk * K + lane - K] = mine;
+    }
+}
+
+// Bits b .. b + 31 of a plane and the 32 after the first (b + 1 .. b + 32).
+// (The planes end in a spare chunk: the word after the last is there.)
+__device__ __forceinline__ void mc_bits33(const uint32_t* plane, uint32_t b, uint32_t& x, uint32_t& x1) {
+    const uint32_t w0 = __ldg(plane + (b >> 5)), w1 = __ldg(plane + (b >> 5) + 1);
+    x = __funnelshift_r(w0, w1, b & 31u);
+    x1 = __funnelshift_rc(w0, w1, (b & 31u) + 1u);   // (a shift of 32 gives w1)
+}
+
+// (1b) mc_bitcount_kernel: a thread takes 32 cubes along x and walks
+// kMcBitRows rows; signs and flags of 32 voxel columns are single words, so a
+// few ANDs and ORs find the cubes with mixed signs and observed corners, and
+// only those look up their triangle counts and are marked in the cubes' own
+// bit plane (linear cube order) for the emission.  The planes (33 MB at 512^3)
+// are read out of L2 (26 us; bound by the instructions of the words that meet
+// the surface).
+constexpr uint32_t kMcBitRows = 4;
+
+template <int MODE>
+__global__ void __launch_bounds__(kMcThreads, 4) mc_bitcount_kernel(const __grid_constant__ McArgs a) {
+    // triangles of the cube whose x-corner nibble is q & 15 and x + 1 nibble q >> 4
+    __shared__ unsigned char s_cnt[256];
+    constexpr int kShift = kMcTileShift[MODE];
+    const uint32_t gx = (uint32_t)a.gx, gy = (uint32_t)a.gy;
+    const uint32_t cx_n = gx - 1, cy_n = gy - 1, cz_n = (uint32_t)a.gz - 1;
+    const uint32_t nseg = (cx_n + 31) / 32, nchunk = (cy_n + kMcBitRows - 1) / kMcBitRows;
+    const uint32_t task = blockIdx.x * blockDim.x + threadIdx.x;   // fewer than voxels
+    const uint32_t rest = task / nseg, cz = rest / nchunk;
+    const bool in = cz < cz_n;
+    const uint32_t x0 = (task - rest * nseg) * 32u;
+    const uint32_t y0 = (rest - cz * nchunk) * kMcBitRows, y1 = min(y0 + kMcBitRows, cy_n);
+    const uint32_t xmask = !in ? 0u : cx_n - x0 >= 32u ? ~0u : (1u << (cx_n - x0)) - 1u;
+    const uint32_t layer = (MODE == kCompat) ? gx + gy : gx * gy;   // marching_cubes.cu:211
+    // voxel row y0 + k in layers z and z + 1 (rows past the grid read the last
+    // one): signs of the 32 columns and of the columns after them, every load
+    // issued before any is used
+    constexpr int K = (int)kMcBitRows;
+    uint32_t p0[K + 1], q0[K + 1], p1[K + 1], q1[K + 1];
+#pragma unroll
+    for (int k = 0; k <= K; ++k) {
+        const uint32_t b = in ? cz * layer + min(y0 + (uint32_t)k, gy - 1u) * gx + x0 : 0u;
+        mc_bits33(a.bits_s, b, p0[k], q0[k]);
+        mc_bits33(a.bits_s, b + layer, p1[k], q1[k]);
+    }
+    uint32_t mixed[K], some = 0u;   // cubes of row y0 + k with both signs
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const uint32_t any = p0[k] | q0[k] | p1[k] | q1[k] | p0[k + 1] | q0[k + 1] | p1[k + 1] | q1[k + 1];
+        const uint32_t all = p0[k] & q0[k] & p1[k] & q1[k] & p0[k + 1] & q0[k + 1] & p1[k + 1] & q1[k + 1];
+        mixed[k] = y0 + (uint32_t)k < y1 ? any & ~all & xmask : 0u;
+        some |= mixed[k];
+    }
+    // few CTAs meet the surface: only those fill the table
+    if (!__syncthreads_or(some != 0u)) return;
+    for (int k = threadIdx.x; k < 256; k += blockDim.x) s_cnt[k] = GBT_MC_TRI_COUNT[mc_type_of_nibbles(k & 15, k >> 4)];
+    __syncthreads();
+    if (!some) return;
+    if (MODE == kFixed) {   // ... and every corner observed
+        uint32_t obs[K + 1];
+#pragma unroll
+        for (int k = 0; k <= K; ++k) {
+            const uint32_t b = cz * layer + min(y0 + (uint32_t)k, gy - 1u) * gx + x0;
+            uint32_t o0, n0, o1, n1;
+            mc_bits33(a.bits_o, b, o0, n0);
+            mc_bits33(a.bits_o, b + layer, o1, n1);
+            obs[k] = o0 & n0 & o1 & n1;
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) mixed[k] &= obs[k] & obs[k + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        uint32_t m = mixed[k];   // (a mixed cube has triangles)
+        if (!m) continue;
+        // the 32 cubes lie in one or two words of 32 (linear order), the
+        // second one possibly in the next tile
+        const uint32_t c0 = (cz * cy_n + y0 + (uint32_t)k) * cx_n + x0;
+        const uint32_t first = 32u - (c0 & 31u), c1 = c0 + first;   // cubes in the first word; the next one
+        const uint32_t m0 = m << (c0 & 31u), m1 = first == 32u ? 0u : m >> first;
+        if (m0) atomicOr(a.cube_bits + (c0 >> 5), m0);
+        if (m1) atomicOr(a.cube_bits + (c1 >> 5), m1);
+        unsigned n0 = 0u, n1 = 0u;
+        for (; m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const uint32_t q = (p0[k] >> j & 1u) | (p1[k] >> j & 1u) << 1 | (p0[k + 1] >> j & 1u) << 2 |
+                               (p1[k + 1] >> j & 1u) << 3 | (q0[k] >> j & 1u) << 4 | (q1[k] >> j & 1u) << 5 |
+                               (q0[k + 1] >> j & 1u) << 6 | (q1[k + 1] >> j & 1u) << 7;
+            if ((uint32_t)j < first) n0 += s_cnt[q]; else n1 += s_cnt[q];
+        }
+        const uint32_t t0 = c0 >> (kShift - 4), t1 = c1 >> (kShift - 4);   // sixteenths of tiles
+        if (t0 == t1) {
+            mc_add_part(a, t0 >> 4, t0 & 15u, n0 + n1);
+        } else {
+            if (n0) mc_add_part(a, t0 >> 4, t0 & 15u, n0);
+            if (n1) mc_add_part(a, t1 >> 4, t1 & 15u, n1);
+        }
+    }
+}
+
 constexpr int kMcScanThreads = 1 << kMcSuperShift;   // one thread per tile of a superblock
 
 // Superblock totals: one CTA per superblock of 1024 tiles sums its tile
-// counts into super[2 sb] (triangles) and super[2 sb + 1] (tiles with
-// triangles).
+// counts into super[2 sb] (triangles) and super[2 sb + 1] (entries of the list
+// of tiles with triangles).
 __global__ void __launch_bounds__(kMcScanThreads) mc_reduce_kernel(const __grid_constant__ McArgs a) {
     __shared__ unsigned long long s_part[kMcScanThreads / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t t = (uint64_t)blockIdx.x * kMcScanThreads + tid;
-    const unsigned long long c = t < a.ntiles ? a.status[t] : 0ull;
-    // packed as the scan packs its sums: triangles << 24 | tiles with triangles
-    unsigned long long v = (c << 24) | (c != 0ull ? 1ull : 0ull);
+    const unsigned c = t < a.ntiles ? mc_tile_triangles(a, t) : 0u;
+    // packed as the scan packs its sums: triangles << 28 | list entries
+    unsigned long long v = ((unsigned long long)c << 28) | mc_tile_entries(a, c);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) s_part[warp] = v;
@@ -1611,18 +1710,18 @@ __global__ void __launch_bounds__(kMcScanThreads) mc_reduce_kernel(const __grid_
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
         if (lane == 0) {
-            a.super[2 * blockIdx.x] = x >> 24;
-            a.super[2 * blockIdx.x + 1] = x & 0xffffffull;
+            a.super[2 * blockIdx.x] = x >> 28;
+            a.super[2 * blockIdx.x + 1] = x & 0xfffffffull;
         }
     }
 }
 
-// Exclusive offsets of the tiles (in place), the list of tiles with
-// triangles, the triangle total and the list length.  One CTA per superblock
-// of 1024 tiles: it sums the totals of the superblocks before it (kept by the
-// count kernel), then scans its own tiles.  Sums travel packed as (triangles
-// << 24 | tiles with triangles): at most 5 * 2^32 triangles and 2^22 tiles,
-// so neither field carries into the other.
+// Exclusive offsets of the tiles (from counts to status, which may be the same
+// words), the list of tiles with triangles (tile | part << 24: part 0 the tile, 1
+// .. 4 a quarter, 5 .. 20 a sixteenth of it), the triangle total and the list length.  One CTA per superblock of 1024
+// tiles: it sums the totals of the superblocks before it, then scans its own
+// tiles.  Sums travel packed as (triangles << 28 | list entries): at most
+// 5 * 2^32 triangles and 2^26 entries, so neither field carries into the other.
 __global__ void __launch_bounds__(kMcScanThreads) mc_scan_kernel(const __grid_constant__ McArgs a) {
     __shared__ unsigned long long s_part[kMcScanThreads / 32];
     __shared__ unsigned long long s_prefix;
@@ -1630,7 +1729,7 @@ __global__ void __launch_bounds__(kMcScanThreads) mc_scan_kernel(const __grid_co
     const uint32_t sb = blockIdx.x;
     // the superblocks before this one
     unsigned long long pre = 0;
-    for (uint32_t k = tid; k < sb; k += kMcScanThreads) pre += (a.super[2 * k] << 24) | a.super[2 * k + 1];
+    for (uint32_t k = tid; k < sb; k += kMcScanThreads) pre += (a.super[2 * k] << 28) | a.super[2 * k + 1];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pre += __shfl_xor_sync(0xffffffffu, pre, o);
     if (lane == 0) s_part[warp] = pre;
@@ -1645,8 +1744,9 @@ __global__ void __launch_bounds__(kMcScanThreads) mc_scan_kernel(const __grid_co
     const unsigned long long prefix = s_prefix;
     // this superblock's tiles, one per thread
     const uint64_t t = (uint64_t)sb * kMcScanThreads + tid;
-    const unsigned long long c = t < a.ntiles ? a.status[t] : 0ull;
-    const unsigned long long own = (c << 24) | (c != 0ull ? 1ull : 0ull);
+    const unsigned c = t < a.ntiles ? mc_tile_triangles(a, t) : 0u;
+    const unsigned entries = mc_tile_entries(a, c);
+    const unsigned long long own = ((unsigned long long)c << 28) | entries;
     unsigned long long x = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1669,13 +1769,16 @@ __global__ void __launch_bounds__(kMcScanThreads) mc_scan_kernel(const __grid_co
     __syncthreads();
     const unsigned long long excl = prefix + s_part[warp] + x - own;
     if (t < a.ntiles) {
-        a.status[t] = excl >> 24;
-        if (c) a.tile_list[excl & 0xffffffull] = (uint32_t)t;
+        a.status[t] = excl >> 28;
+        uint32_t* e = a.tile_list + (excl & 0xfffffffull);
+        if (entries == 1u) e[0] = (uint32_t)t;
+        if (entries > 1u)
+            for (uint32_t q = 0; q < entries; ++q) e[q] = (uint32_t)t | ((entries == 4u ? 1u : 5u) + q) << 24;
     }
     if (sb == gridDim.x - 1 && tid == kMcScanThreads - 1) {
         const unsigned long long all = excl + own;
-        *a.total = (long long)(all >> 24);
-        *a.nonempty = (unsigned)(all & 0xffffffull);
+        *a.total = (long long)(all >> 28);
+        *a.nonempty = (unsigned)(all & 0xfffffffull);
     }
 }
 
@@ -1748,36 +1851,78 @@ __device__ __forceinline__ int32_t mc_vertex_index(const McArgs& a, uint32_t cx,
     return (int32_t)(a.index_base + a.edge_word_offset[id >> 5] + __popc(below));
 }
 
+// A warp's rings of queued cubes and triangles, and their output.
 template <int MODE>
-__global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_constant__ McArgs a) {
-    constexpr int kWarps = kMcThreads / 32;
-    __shared__ unsigned char s_count[256];
-    __shared__ unsigned long long s_tri[256];
-    __shared__ unsigned char s_ends[12];
-    __shared__ unsigned char s_type[256];
-    __shared__ float s_cval[kWarps][8][kMcCubeRing];        // corner values of the queued cubes
-    __shared__ uint32_t s_cube[kWarps][kMcCubeRing];         // their linear index
-    __shared__ unsigned char s_ctype[kWarps][kMcCubeRing];   // their case
-    __shared__ unsigned short s_tq[kWarps][kMcTriRing];      // queued triangles: cube slot | triangle << 6
-    __shared__ float s_out[kWarps][32 * 9];                  // a batch of 32 triangles
-    mc_load_tables(s_count, s_tri, s_ends, s_type);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned njobs = *a.nonempty;
-    constexpr uint32_t kWords = (uint32_t)mc_tile_cubes(MODE) / 1024u;   // group words per tile
-    const uint32_t nwords = (a.ncubes + 1023u) / 1024u;
-    const bool indexed = MODE == kFixed && a.edge_bits != nullptr;
-    float (*cval)[kMcCubeRing] = s_cval[warp];
-    uint32_t* cube_of = s_cube[warp];
-    unsigned char* ctype = s_ctype[warp];
-    unsigned short* tq = s_tq[warp];
-    float* sout = s_out[warp];
+struct McEmitRings {
+    const McArgs& a;
+    float (*cval)[kMcCubeRing];
+    uint32_t* cube_of;
+    unsigned char* ctype;
+    unsigned short* tq;
+    float* sout;
+    const unsigned char* s_count;
+    const unsigned long long* s_tri;
+    const unsigned char* s_ends;
+    int lane;
+    bool indexed;
+    uint32_t tq_head, tq_tail, cq_head;   // (the same in every lane, as is out_next)
+    long long out_next;                   // the next triangle to write
 
-    // writes the queued triangles [head, head + cnt) (cnt <= 32) from output `first`
-    auto emit_batch = [&](uint32_t head, int cnt, long long first) {
-        const bool act = lane < cnt;
-        if (act) {
-            const unsigned e16 = tq[(head + (uint32_t)lane) & (kMcTriRing - 1)];
+    __device__ __forceinline__ void begin(long long first) {
+        tq_head = tq_tail = cq_head = 0u;
+        out_next = first;
+    }
+
+    // Queues the lanes' cubes that have triangles (case `type`, 0: none; lanes in
+    // cube order; X: corners 0, 3, 4, 7, N: 1, 2, 5, 6) and writes the full
+    // batches of 32 triangles.
+    __device__ __forceinline__ void push(uint32_t c, const float (&X)[4], const float (&N)[4], int type) {
+        const int n = s_count[type];
+        // the cubes with triangles take consecutive ring slots
+        const uint32_t act = __ballot_sync(0xffffffffu, n > 0);
+        const uint32_t rank = (uint32_t)__popc(act & ((1u << lane) - 1u));
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        if (n > 0) {
+            const int sl = (int)((cq_head + rank) & (kMcCubeRing - 1));
+            // the cube's eight corners in the reference's numbering
+            cval[0][sl] = X[0];
+            cval[1][sl] = N[0];
+            cval[2][sl] = N[1];
+            cval[3][sl] = X[1];
+            cval[4][sl] = X[2];
+            cval[5][sl] = N[2];
+            cval[6][sl] = N[3];
+            cval[7][sl] = X[3];
+            cube_of[sl] = c;
+            ctype[sl] = (unsigned char)type;
+            for (int k = 0; k < n; ++k)
+                tq[(tq_tail + (uint32_t)(incl - n + k)) & (kMcTriRing - 1)] = (unsigned short)(sl | k << 6);
+        }
+        cq_head += (uint32_t)__popc(act);
+        tq_tail += (uint32_t)total;
+        __syncwarp();
+        while (tq_tail - tq_head >= 32u) {
+            write(32);
+            tq_head += 32u;
+            out_next += 32;
+        }
+    }
+
+    __device__ __forceinline__ void finish() {
+        if (tq_tail != tq_head) write((int)(tq_tail - tq_head));
+    }
+
+    // writes the queued triangles [tq_head, tq_head + cnt) (cnt <= 32) from output out_next
+    __device__ __forceinline__ void write(int cnt) {
+        const long long first = out_next;
+        if (lane < cnt) {
+            const unsigned e16 = tq[(tq_head + (uint32_t)lane) & (kMcTriRing - 1)];
             const int sl = (int)(e16 & 63u), tr = (int)(e16 >> 6);
             const uint32_t cc = cube_of[sl];
             const int t = ctype[sl];
@@ -1811,7 +1956,30 @@ __global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_consta
             for (int f = lane; f < nf / 3; f += 32) a.tris[3 * first + f] = (int32_t)(a.index_base + 3 * first + f);
         }
         __syncwarp();
-    };
+    }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_constant__ McArgs a) {
+    constexpr int kWarps = kMcThreads / 32;
+    __shared__ unsigned char s_count[256];
+    __shared__ unsigned long long s_tri[256];
+    __shared__ unsigned char s_ends[12];
+    __shared__ unsigned char s_type[256];
+    __shared__ float s_cval[kWarps][8][kMcCubeRing];        // corner values of the queued cubes
+    __shared__ uint32_t s_cube[kWarps][kMcCubeRing];         // their linear index
+    __shared__ unsigned char s_ctype[kWarps][kMcCubeRing];   // their case
+    __shared__ unsigned short s_tq[kWarps][kMcTriRing];      // queued triangles: cube slot | triangle << 6
+    __shared__ float s_out[kWarps][32 * 9];                  // a batch of 32 triangles
+    mc_load_tables(s_count, s_tri, s_ends, s_type);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned njobs = *a.nonempty;
+    constexpr uint32_t kWords = (uint32_t)mc_tile_cubes(MODE) / 1024u;   // group words per tile
+    const uint32_t nwords = (a.ncubes + 1023u) / 1024u;
+    const bool indexed = MODE == kFixed && a.edge_bits != nullptr;
+    McEmitRings<MODE> R{a, s_cval[warp], s_cube[warp], s_ctype[warp], s_tq[warp], s_out[warp], s_count, s_tri,
+                        s_ends, lane, indexed, 0u, 0u, 0u, 0ll};
 
     for (;;) {
         unsigned job = 0;
@@ -1819,8 +1987,7 @@ __global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_consta
         job = __shfl_sync(0xffffffffu, job, 0);
         if (job >= njobs) break;
         const uint32_t tile = a.tile_list[job];
-        long long out_next = (long long)a.status[tile];   // this tile's next triangle to write
-        uint32_t tq_head = 0, tq_tail = 0, cq_head = 0;  // (the same in every lane)
+        R.begin((long long)a.status[tile]);   // the tile's first triangle
 #pragma unroll 1
         for (uint32_t w = 0; w < kWords; ++w) {
             const uint32_t word = tile * kWords + w;
@@ -1864,44 +2031,135 @@ __global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_consta
                 }
                 int type = s_type[sx | sn << 4];
                 if (!in || (MODE == kFixed && !(okx && okn))) type = 0;
-                const int n = s_count[type];
-                // the cubes with triangles take consecutive ring slots, in cube order
-                const uint32_t act = __ballot_sync(0xffffffffu, n > 0);
-                const uint32_t rank = (uint32_t)__popc(act & ((1u << lane) - 1u));
-                int incl = n;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                if (n > 0) {
-                    const int sl = (int)((cq_head + rank) & (kMcCubeRing - 1));
-                    // the cube's eight corners in the reference's numbering
-                    cval[0][sl] = X[0];
-                    cval[1][sl] = N[0];
-                    cval[2][sl] = N[1];
-                    cval[3][sl] = X[1];
-                    cval[4][sl] = X[2];
-                    cval[5][sl] = N[2];
-                    cval[6][sl] = N[3];
-                    cval[7][sl] = X[3];
-                    cube_of[sl] = c;
-                    ctype[sl] = (unsigned char)type;
-                    for (int k = 0; k < n; ++k)
-                        tq[(tq_tail + (uint32_t)(incl - n + k)) & (kMcTriRing - 1)] = (unsigned short)(sl | k << 6);
-                }
-                cq_head += (uint32_t)__popc(act);
-                tq_tail += (uint32_t)total;
-                __syncwarp();
-                while (tq_tail - tq_head >= 32u) {
-                    emit_batch(tq_head, 32, out_next);
-                    tq_head += 32u;
-                    out_next += 32;
-                }
+                R.push(c, X, N, type);
             }
         }
-        if (tq_tail != tq_head) emit_batch(tq_head, (int)(tq_tail - tq_head), out_next);
+        R.finish();
+    }
+}
+
+// Emission from the cubes' bit plane (cube_bits): a warp takes entries of the
+// list of tiles, gathers an entry's marked cubes 32 at a time, one per lane,
+// loads the eight corners of each, and writes triangles as mc_emit_kernel does.
+// Taking the marked cubes from the plane instead of classifying every cube of a
+// marked group of 32 again fills the lanes (a group on a surface has some five
+// cubes with triangles) and reads no weights: 19 M instead of 41 M warp
+// instructions for 870 K triangles at 512^3, 70 us against 82 (35 against 54 at
+// 384^3 as indices).  Bound by the chain of loads from list to corners and its
+// own instructions; the first links of the chain are read ahead.
+constexpr int kMcEmitThreads = 128;
+
+template <int MODE>
+__global__ void __launch_bounds__(kMcEmitThreads) mc_emit_cubes_kernel(const __grid_constant__ McArgs a) {
+    constexpr int kWarps = kMcEmitThreads / 32;
+    __shared__ unsigned char s_count[256];
+    __shared__ unsigned long long s_tri[256];
+    __shared__ unsigned char s_ends[12];
+    __shared__ unsigned char s_type[256];
+    __shared__ float s_cval[kWarps][8][kMcCubeRing];        // corner values of the queued cubes
+    __shared__ uint32_t s_cube[kWarps][kMcCubeRing];         // their linear index
+    __shared__ unsigned char s_ctype[kWarps][kMcCubeRing];   // their case
+    __shared__ unsigned short s_tq[kWarps][kMcTriRing];      // queued triangles: cube slot | triangle << 6
+    __shared__ float s_out[kWarps][32 * 9];                  // a batch of 32 triangles
+    __shared__ unsigned short s_list[kWarps][1024];          // marked cubes of 32 words, numbered from the first word's
+    const unsigned njobs = *a.nonempty;
+    if ((unsigned)blockIdx.x * kWarps >= njobs) return;   // more warps than entries
+    mc_load_tables(s_count, s_tri, s_ends, s_type);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr uint32_t kTileWords = (uint32_t)mc_tile_cubes(MODE) / 32u;   // of 32 cubes
+    const uint32_t nwords = (a.ncubes + 31u) / 32u;
+    const bool indexed = MODE == kFixed && a.edge_bits != nullptr;
+    McEmitRings<MODE> R{a, s_cval[warp], s_cube[warp], s_ctype[warp], s_tq[warp], s_out[warp], s_count, s_tri,
+                        s_ends, lane, indexed, 0u, 0u, 0u, 0ll};
+    unsigned short* list = s_list[warp];
+    // loads the corners of one marked cube per lane (`in` false: none) and queues it
+    auto take = [&](uint32_t c, bool in) {
+        uint32_t idx[4];
+        cube_xcorners<MODE>(a, in ? c : 0u, idx);
+        float X[4], N[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            X[k] = __ldg(a.D + idx[k]);
+            N[k] = __ldg(a.D + idx[k] + 1);
+        }
+        int sx = 0, sn = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            sx |= (X[k] < 0.f) << k;
+            sn |= (N[k] < 0.f) << k;
+        }
+        R.push(c, X, N, in ? s_type[sx | sn << 4] : 0);
+    };
+    // The warp's entries are gw, gw + nw, ...: an entry is read two entries
+    // before its cubes are taken, its offset and marked cubes one before.
+    constexpr int kRounds = (int)kTileWords / 32;
+    struct Entry {
+        uint32_t w0, w1;          // its words: the tile's, or a quarter or sixteenth of them
+        uint32_t bits[kRounds];   // the lane's words
+        long long first;          // its first triangle
+    };
+    auto fetch = [&](uint32_t e) {
+        Entry r;
+        const uint32_t t = e & 0xffffffu, part = e >> 24;
+        const uint32_t p0 = part == 0u ? 0u : part <= 4u ? 4u * (part - 1u) : part - 5u;   // its first sixteenth
+        const uint32_t np = part == 0u ? 16u : part <= 4u ? 4u : 1u;
+        r.w0 = t * kTileWords + p0 * (kTileWords / 16u);
+        r.w1 = min(r.w0 + np * (kTileWords / 16u), nwords);
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            const uint32_t w = r.w0 + 32u * k + (uint32_t)lane;
+            r.bits[k] = w < r.w1 ? __ldg(a.cube_bits + w) : 0u;
+        }
+        r.first = (long long)a.status[t];
+        if (p0) {   // the triangles of the sixteenths before it
+            const unsigned n = (uint32_t)lane < p0 ? reinterpret_cast<const unsigned short*>(a.counts + 4ull * t)[lane] : 0u;
+            r.first += __reduce_add_sync(0xffffffffu, n);
+        }
+        return r;
+    };
+    const uint32_t nw = gridDim.x * kWarps;
+    uint32_t job = blockIdx.x * kWarps + (uint32_t)warp;
+    if (job >= njobs) return;
+    Entry next = fetch(a.tile_list[job]);
+    uint32_t after = job + nw < njobs ? a.tile_list[job + nw] : 0u;
+    for (; job < njobs; job += nw) {
+        const Entry cur = next;
+        if (job + nw < njobs) next = fetch(after);
+        if (job + nw < njobs && job + 2u * nw < njobs) after = a.tile_list[job + 2u * nw];
+        R.begin(cur.first);
+        uint32_t pending = 0u, held = 0u;   // lanes below `held` hold a marked cube that has not been queued yet
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+            uint32_t bits = cur.bits[k];
+            const uint32_t n = (uint32_t)__popc(bits);
+            uint32_t incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            if (total == 0u) continue;
+            for (uint32_t at = incl - n; bits; bits &= bits - 1u)
+                list[at++] = (unsigned short)(32u * (uint32_t)lane + (uint32_t)__ffs(bits) - 1u);
+            __syncwarp();
+            const uint32_t first = (cur.w0 + 32u * k) * 32u;
+            uint32_t taken = 0u;   // of the list
+            while (held + total - taken >= 32u) {
+                const uint32_t c = (uint32_t)lane < held ? pending : first + list[taken + (uint32_t)lane - held];
+                taken += 32u - held;
+                held = 0u;
+                take(c, true);
+            }
+            const uint32_t left = total - taken;   // held + left < 32
+            if ((uint32_t)lane >= held && (uint32_t)lane < held + left)
+                pending = first + list[taken + (uint32_t)lane - held];
+            held += left;
+            __syncwarp();   // the list may be written again
+        }
+        if (held) take(pending, (uint32_t)lane < held);
+        R.finish();
     }
 }
 
@@ -2205,7 +2463,7 @@ int resident_ctas_mode(int kind, int brick) {
 // The three marching-cubes launches; the scratch words (total, list length,
 // tile words, group bits) are zero when the first starts.
 struct McGrid {
-    int sms, per_count, per_count4, per_emit;
+    int sms, per_count, per_count4, per_bits, per_emit, per_cubes;
 };
 
 // SMs and resident CTAs of the count and emit kernels (thread-safe
@@ -2213,17 +2471,21 @@ struct McGrid {
 template <int MODE>
 const McGrid& mc_grid() {
     static const McGrid g = [] {
-        McGrid r{1, 1, 1, 1};
+        McGrid r{1, 1, 1, 1, 1, 1};
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_count, mc_count_kernel<MODE>, kMcThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_count4, mc_count4_kernel<MODE>, kMcThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_bits, mc_bits_kernel<MODE>, kMcThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_emit, mc_emit_kernel<MODE>, kMcThreads, 0);
         cudaGetLastError();
         if (r.sms < 1) r.sms = 1;
         if (r.per_count < 1) r.per_count = 1;
         if (r.per_count4 < 1) r.per_count4 = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_cubes, mc_emit_cubes_kernel<MODE>, kMcEmitThreads, 0);
+        if (r.per_cubes < 1) r.per_cubes = 1;
+        if (r.per_bits < 1) r.per_bits = 1;
         if (r.per_emit < 1) r.per_emit = 1;
         return r;
     }();
@@ -2237,8 +2499,22 @@ bool mc_rows_of_4(const McArgs& a) {
            (MODE == kCompat || (reinterpret_cast<uintptr_t>(a.W) & 15u) == 0);
 }
 
+// Counts from bit planes: the planes, then the cubes.
 template <int MODE>
-cudaError_t launch_mc_mode(const McArgs& a, cudaStream_t s) {
+void launch_mc_bitcount(const McArgs& a, cudaStream_t s) {
+    const McGrid& mg = mc_grid<MODE>();
+    long long grid = (long long)mg.sms * mg.per_bits;
+    const long long need = ((long long)mc_bit_chunks(a.nbits) + kMcThreads / 32 - 1) / (kMcThreads / 32);
+    if (grid > need) grid = need;
+    mc_bits_kernel<MODE><<<(int)grid, kMcThreads, 0, s>>>(a);
+    const long long nseg = (a.gx - 1 + 31) / 32, nchunk = (a.gy - 1 + (long long)kMcBitRows - 1) / kMcBitRows;
+    const long long ntasks = nseg * nchunk * (a.gz - 1);
+    mc_bitcount_kernel<MODE><<<(unsigned)((ntasks + kMcThreads - 1) / kMcThreads), kMcThreads, 0, s>>>(a);
+}
+
+// Counts by row walks over the distances and weights (no bit planes).
+template <int MODE>
+void launch_mc_rowcount(const McArgs& a, cudaStream_t s) {
     const McGrid& mg = mc_grid<MODE>();
     const bool four = mc_rows_of_4<MODE>(a);
     // one warp per task (a segment of a cube layer, a run of rows)
@@ -2255,15 +2531,28 @@ cudaError_t launch_mc_mode(const McArgs& a, cudaStream_t s) {
         mc_count4_kernel<MODE><<<(int)grid, kMcThreads, 0, s>>>(a);
     else
         mc_count_kernel<MODE><<<(int)grid, kMcThreads, 0, s>>>(a);
+}
+
+template <int MODE>
+cudaError_t launch_mc_mode(const McArgs& a, cudaStream_t s) {
+    const McGrid& mg = mc_grid<MODE>();
+    if (a.bits_s)
+        launch_mc_bitcount<MODE>(a, s);
+    else
+        launch_mc_rowcount<MODE>(a, s);
     const unsigned nsuper = (unsigned)((a.ntiles + kMcScanThreads - 1) / kMcScanThreads);
     mc_reduce_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
     mc_scan_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
-    grid = (long long)mg.sms * mg.per_emit;
-    const long long tiles_per_cta = kMcThreads / 32;   // a warp per listed tile at least
+    const int threads = a.bits_s ? kMcEmitThreads : kMcThreads;
+    long long grid = (long long)mg.sms * (a.bits_s ? mg.per_cubes : mg.per_emit);
+    const long long tiles_per_cta = threads / 32;   // a warp per listed tile at least
     if (grid > ((long long)a.ntiles + tiles_per_cta - 1) / tiles_per_cta)
         grid = ((long long)a.ntiles + tiles_per_cta - 1) / tiles_per_cta;
     if (grid < 1) grid = 1;
-    mc_emit_kernel<MODE><<<(int)grid, kMcThreads, 0, s>>>(a);
+    if (a.bits_s)
+        mc_emit_cubes_kernel<MODE><<<(int)grid, threads, 0, s>>>(a);
+    else
+        mc_emit_kernel<MODE><<<(int)grid, threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -117,7 +117,8 @@ gbt_status gbt_extract_mesh_noalloc(gbt_volume* v, float* verts, int32_t* tris, 
     a.nonempty = reinterpret_cast<unsigned int*>(s + 16);
     const size_t nsuper = (size_t)gbt::mc_superblocks(a.ntiles);
     a.super = reinterpret_cast<unsigned long long*>(s + 64);
-    a.status = a.super + 2 * nsuper;
+    a.counts = a.super + 2 * nsuper;
+    a.status = a.counts;   // offsets in place
     const size_t nwords = (size_t)gbt::mc_group_words(ncubes);
     a.group_bits = reinterpret_cast<uint32_t*>(a.status + a.ntiles);
     a.tile_list = a.group_bits + nwords;
