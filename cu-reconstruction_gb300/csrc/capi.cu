@@ -718,21 +718,44 @@ gbt_status mc_prepare(gbt_volume* v, float* verts, int32_t* tris, int64_t cap, i
     return GBT_OK;
 }
 
-gbt_status mc_launch(gbt_volume* v, const gbt::McArgs& a, cudaStream_t s) {
+// The launches of `phases` (a mesh without room, a.cap 0, has nothing to emit).
+gbt_status mc_launch(gbt_volume* v, const gbt::McArgs& a, cudaStream_t s,
+                     int phases = gbt::kMcCount | gbt::kMcEmit) {
     cudaGetLastError();  // a launch reports only its own failure
+    if (a.cap == 0) phases &= ~gbt::kMcEmit;
+    cudaError_t e = cudaSuccess;
     // header, superblock totals, tile words and cube bits start at zero
-    cudaError_t e = cudaMemsetAsync(v->mc_scratch, 0,
+    if (phases & gbt::kMcCount)
+        e = cudaMemsetAsync(v->mc_scratch, 0,
                                     64 + (size_t)gbt::mc_superblocks(a.ntiles) * 16 + (size_t)a.ntiles * 32 +
                                         ((size_t)a.ncubes + 31) / 32 * 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "mesh scratch clear");
     if (a.ntiles == 0) return GBT_OK;
     if (v->cfg.mode == GBT_MODE_FIXED)
-        e = gbt::launch_mc_fixed(a, s);
+        e = gbt::launch_mc_fixed(a, phases, s);
     else if (v->cfg.arith == GBT_ARITH_IEEE)
-        e = gbt::launch_mc_compat_ieee(a, s);
+        e = gbt::launch_mc_compat_ieee(a, phases, s);
     else
-        e = gbt::launch_mc_compat_ref(a, s);
+        e = gbt::launch_mc_compat_ref(a, phases, s);
     if (e != cudaSuccess) return cuda_fail(e, "mesh launch");
+    return GBT_OK;
+}
+
+// The head of the mesh scratch, as the kernels leave it.
+struct McHeader {
+    unsigned int ticket;
+    int error;
+    long long total;
+    unsigned int entries, pad;
+    long long nverts;   // shared vertices, written by their numbering
+};
+
+// Waits for `s` and reads the header.
+gbt_status mc_read_header(gbt_volume* v, McHeader* hdr, cudaStream_t s) {
+    cudaError_t e = cudaMemcpyAsync(hdr, v->mc_scratch, sizeof(*hdr), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(e, "mesh extraction");
+    if (hdr->error) return fail(GBT_ERR_CUDA, "mesh extraction: the kernels set their error word");
     return GBT_OK;
 }
 
@@ -751,15 +774,9 @@ gbt_status gbt_extract_mesh(gbt_volume* v, float* verts, int32_t* tris, int64_t 
     cudaStream_t s = as_stream(stream);
     st = mc_launch(v, a, s);
     if (st != GBT_OK) return st;
-    struct {
-        unsigned int ticket;
-        int error;
-        long long total;
-    } hdr;
-    cudaError_t e = cudaMemcpyAsync(&hdr, v->mc_scratch, sizeof(hdr), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(e, "mesh extraction");
-    if (hdr.error) return fail(GBT_ERR_CUDA, "mesh extraction: the kernels set their error word");
+    McHeader hdr;
+    st = mc_read_header(v, &hdr, s);
+    if (st != GBT_OK) return st;
     *n_tris = hdr.total;
     if (hdr.total > cap_tris && cap_tris > 0)
         return fail(GBT_ERR_CAPACITY, "mesh has %lld triangles, buffer holds %lld", hdr.total, (long long)cap_tris);
@@ -1081,28 +1098,16 @@ gbt_status gbt_diff_backward(const gbt_diff_cfg* cfg, const void* grad_tsdf, con
     return GBT_OK;
 }
 
-gbt_status gbt_extract_mesh_indexed(gbt_volume* v, float* verts, float* normals, int32_t* tris, int64_t cap_verts,
-                                    int64_t cap_tris, int64_t index_base, int64_t* n_verts, int64_t* n_tris,
-                                    void* stream) {
-    gbt::TraceRange trace_("gbt_extract_mesh_indexed");
-    if (!n_verts || !n_tris) return fail(GBT_ERR_INVALID_ARG, "gbt_extract_mesh_indexed: n_verts or n_tris is NULL");
-    *n_verts = 0;
-    *n_tris = 0;
-    if (!v) return fail(GBT_ERR_INVALID_ARG, "volume is NULL");
-    if (v->cfg.mode != GBT_MODE_FIXED)
-        return fail(GBT_ERR_INVALID_ARG,
-                    "gbt_extract_mesh_indexed: fixed mode only (compat emits three vertices per triangle, as the "
-                    "reference does)");
-    if (cap_verts < 0 || (cap_verts > 0 && !verts)) return fail(GBT_ERR_INVALID_ARG, "vertex buffer is NULL");
-    gbt::McArgs a;
-    gbt_status st = mc_prepare(v, nullptr, tris, cap_tris, index_base, &a, true);
-    if (st != GBT_OK) return st;
-    const gbt::VolDesc& d = v->desc;
-    gbt::WeldArgs w;
-    std::memset(&w, 0, sizeof(w));
-    w.nwords = (3 * v->nvox + 31) / 32;
-    w.nblocks = (w.nwords + gbt::kWeldWordsPerBlock - 1) / gbt::kWeldWordsPerBlock;
-    const size_t need = 64 + (size_t)w.nwords * 8 + (size_t)w.nblocks * 4;
+}  // extern "C"
+
+namespace {
+
+// Scratch and arguments of the shared-vertex numbering.
+gbt_status weld_prepare(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w) {
+    std::memset(w, 0, sizeof(*w));
+    w->nwords = (3 * v->nvox + 31) / 32;
+    w->nblocks = (w->nwords + gbt::kWeldWordsPerBlock - 1) / gbt::kWeldWordsPerBlock;
+    const size_t need = (size_t)w->nwords * 8 + (size_t)w->nblocks * 4;
     if (v->weld_scratch_bytes < need) {
         if (v->weld_scratch) cudaFree(v->weld_scratch);
         v->weld_scratch = nullptr;
@@ -1114,50 +1119,140 @@ gbt_status gbt_extract_mesh_indexed(gbt_volume* v, float* verts, float* normals,
         }
         v->weld_scratch_bytes = need;
     }
-    char* sp = static_cast<char*>(v->weld_scratch);
-    w.nverts = reinterpret_cast<long long*>(sp);
-    w.bits = reinterpret_cast<uint32_t*>(sp + 64);
-    w.word_offset = w.bits + w.nwords;
-    w.block_sums = w.word_offset + w.nwords;
-    (void)d;
-    cudaStream_t s = as_stream(stream);
-    cudaGetLastError();
-    cudaError_t e = cudaMemsetAsync(w.bits, 0, (size_t)w.nwords * 4, s);
-    if (e != cudaSuccess) return cuda_fail(e, "vertex-sharing scratch clear");
-    w.mc = a;
-    e = gbt::launch_weld_fixed(w, s);
-    if (e != cudaSuccess) return cuda_fail(e, "edge marking");
-    long long nv = 0;
-    e = cudaMemcpyAsync(&nv, w.nverts, sizeof(nv), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(e, "vertex count");
-    if (nv > (long long)INT32_MAX - (index_base > 0 ? index_base : 0))
-        return fail(GBT_ERR_INVALID_ARG, "%lld vertices do not fit 32-bit triangle indices", nv);
-    *n_verts = nv;
+    w->nverts = &reinterpret_cast<McHeader*>(v->mc_scratch)->nverts;
+    w->bits = static_cast<uint32_t*>(v->weld_scratch);
+    w->word_offset = w->bits + w->nwords;
+    w->block_sums = w->word_offset + w->nwords;
+    w->mc = a;
+    return GBT_OK;
+}
+
+// Counts triangles and, with w, numbers the shared vertices; returns the totals.
+gbt_status mc_count(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w, McHeader* hdr, cudaStream_t s) {
+    gbt_status st = mc_launch(v, a, s, gbt::kMcCount);
+    if (st != GBT_OK) return st;
+    if (w) {
+        cudaError_t e = cudaMemsetAsync(w->bits, 0, (size_t)w->nwords * 4, s);
+        if (e != cudaSuccess) return cuda_fail(e, "vertex-sharing scratch clear");
+        e = gbt::launch_weld_fixed(*w, s);
+        if (e != cudaSuccess) return cuda_fail(e, "edge marking");
+    }
+    return mc_read_header(v, hdr, s);
+}
+
+// Writes the vertices and normals, and the triangles as their indices.
+gbt_status mc_emit_indexed(gbt_volume* v, gbt::McArgs a, gbt::WeldArgs& w, float* verts, float* normals,
+                           int64_t cap_verts, cudaStream_t s) {
     if (verts && cap_verts > 0) {
         w.verts = verts;
         w.normals = normals;
         w.cap_verts = cap_verts;
-        e = gbt::launch_weld_vertices_fixed(w, s);
+        cudaError_t e = gbt::launch_weld_vertices_fixed(w, s);
         if (e != cudaSuccess) return cuda_fail(e, "vertices");
     }
     a.edge_bits = w.bits;
     a.edge_word_offset = w.word_offset;
-    st = mc_launch(v, a, s);
+    return mc_launch(v, a, s, gbt::kMcEmit);
+}
+
+gbt_status weld_count_fits(long long nv, int64_t index_base) {
+    if (nv > (long long)INT32_MAX - (index_base > 0 ? index_base : 0))
+        return fail(GBT_ERR_INVALID_ARG, "%lld vertices do not fit 32-bit triangle indices", nv);
+    return GBT_OK;
+}
+
+gbt_status weld_mode_ok(const gbt_volume* v, const char* fn) {
+    if (!v) return fail(GBT_ERR_INVALID_ARG, "volume is NULL");
+    if (v->cfg.mode != GBT_MODE_FIXED)
+        return fail(GBT_ERR_INVALID_ARG,
+                    "%s: fixed mode only (compat emits three vertices per triangle, as the reference does)", fn);
+    return GBT_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+gbt_status gbt_extract_mesh_indexed(gbt_volume* v, float* verts, float* normals, int32_t* tris, int64_t cap_verts,
+                                    int64_t cap_tris, int64_t index_base, int64_t* n_verts, int64_t* n_tris,
+                                    void* stream) {
+    gbt::TraceRange trace_("gbt_extract_mesh_indexed");
+    if (!n_verts || !n_tris) return fail(GBT_ERR_INVALID_ARG, "gbt_extract_mesh_indexed: n_verts or n_tris is NULL");
+    *n_verts = 0;
+    *n_tris = 0;
+    gbt_status st = weld_mode_ok(v, "gbt_extract_mesh_indexed");
     if (st != GBT_OK) return st;
-    struct {
-        unsigned int ticket;
-        int error;
-        long long total;
-    } hdr;
-    e = cudaMemcpyAsync(&hdr, v->mc_scratch, sizeof(hdr), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (cap_verts < 0 || (cap_verts > 0 && !verts)) return fail(GBT_ERR_INVALID_ARG, "vertex buffer is NULL");
+    gbt::McArgs a;
+    st = mc_prepare(v, nullptr, tris, cap_tris, index_base, &a, true);
+    if (st != GBT_OK) return st;
+    gbt::WeldArgs w;
+    st = weld_prepare(v, a, &w);
+    if (st != GBT_OK) return st;
+    cudaStream_t s = as_stream(stream);
+    McHeader hdr;
+    st = mc_count(v, a, &w, &hdr, s);
+    if (st != GBT_OK) return st;
+    st = weld_count_fits(hdr.nverts, index_base);
+    if (st != GBT_OK) return st;
+    *n_verts = hdr.nverts;
+    st = mc_emit_indexed(v, a, w, verts, normals, cap_verts, s);
+    if (st != GBT_OK) return st;
+    cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e, "mesh extraction");
-    if (hdr.error) return fail(GBT_ERR_CUDA, "mesh extraction: the kernels set their error word");
     *n_tris = hdr.total;
-    if ((hdr.total > cap_tris && cap_tris > 0) || (nv > cap_verts && cap_verts > 0))
-        return fail(GBT_ERR_CAPACITY, "mesh has %lld vertices and %lld triangles, buffers hold %lld and %lld", nv,
-                    hdr.total, (long long)cap_verts, (long long)cap_tris);
+    if ((hdr.total > cap_tris && cap_tris > 0) || (hdr.nverts > cap_verts && cap_verts > 0))
+        return fail(GBT_ERR_CAPACITY, "mesh has %lld vertices and %lld triangles, buffers hold %lld and %lld",
+                    hdr.nverts, hdr.total, (long long)cap_verts, (long long)cap_tris);
+    return GBT_OK;
+}
+
+gbt_status gbt_extract_mesh_sized(gbt_volume* v, int32_t shared_vertices, gbt_mesh_alloc alloc, void* ctx,
+                                  int64_t index_base, int64_t* n_verts, int64_t* n_tris, void* stream) {
+    gbt::TraceRange trace_("gbt_extract_mesh_sized");
+    if (!n_verts || !n_tris || !alloc)
+        return fail(GBT_ERR_INVALID_ARG, "gbt_extract_mesh_sized: alloc, n_verts or n_tris is NULL");
+    *n_verts = 0;
+    *n_tris = 0;
+    const bool shared = shared_vertices != 0;
+    gbt_status st = shared ? weld_mode_ok(v, "gbt_extract_mesh_sized") : GBT_OK;
+    if (st != GBT_OK) return st;
+    gbt::McArgs a;
+    st = mc_prepare(v, nullptr, nullptr, 0, index_base, &a, shared);
+    if (st != GBT_OK) return st;
+    gbt::WeldArgs w;
+    if (shared) {
+        st = weld_prepare(v, a, &w);
+        if (st != GBT_OK) return st;
+    }
+    cudaStream_t s = as_stream(stream);
+    McHeader hdr;
+    st = mc_count(v, a, shared ? &w : nullptr, &hdr, s);
+    if (st != GBT_OK) return st;
+    if (shared) {
+        st = weld_count_fits(hdr.nverts, index_base);
+        if (st != GBT_OK) return st;
+    } else if (!gbt::mc_indices_fit(hdr.total, index_base)) {
+        return fail(GBT_ERR_INVALID_ARG, "index_base %lld + 3 x %lld triangles passes the int32 index range",
+                    (long long)index_base, hdr.total);
+    }
+    const int64_t nv = shared ? hdr.nverts : 3 * hdr.total;
+    float *verts = nullptr, *normals = nullptr;
+    int32_t* tris = nullptr;
+    if (alloc(ctx, nv, hdr.total, &verts, &normals, &tris) != 0)
+        return fail(GBT_ERR_ALLOC, "gbt_extract_mesh_sized: no buffers for %lld triangles", hdr.total);
+    if (hdr.total > 0) {
+        if (!verts || !tris) return fail(GBT_ERR_INVALID_ARG, "output buffers are NULL");
+        a.verts = verts;
+        a.tris = tris;
+        a.cap = hdr.total;
+        st = shared ? mc_emit_indexed(v, a, w, verts, normals, nv, s) : mc_launch(v, a, s, gbt::kMcEmit);
+        if (st != GBT_OK) return st;
+        cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return cuda_fail(e, "mesh extraction");
+    }
+    *n_verts = nv;
+    *n_tris = hdr.total;
     return GBT_OK;
 }
 

@@ -251,12 +251,14 @@ struct DiffArgs {
 // Launchers exported by the kernel translation units.
 // k_ref.cu (-use_fast_math): compat mode in the reference's arithmetic.
 cudaError_t launch_integrate_compat_ref(const IntegrateArgs& a, int brick, int grid, cudaStream_t s);
-cudaError_t launch_mc_compat_ref(const McArgs& a, cudaStream_t s);
+// (marching cubes: the launches of `phases`, counts and offsets or the emission from them)
+enum { kMcCount = 1, kMcEmit = 2 };
+cudaError_t launch_mc_compat_ref(const McArgs& a, int phases, cudaStream_t s);
 // k_ieee.cu (IEEE arithmetic): compat mode as the oracle computes it, fixed mode.
 cudaError_t launch_integrate_compat_ieee(const IntegrateArgs& a, int brick, int grid, cudaStream_t s);
 cudaError_t launch_integrate_fixed(const IntegrateArgs& a, int brick, int grid, cudaStream_t s);
-cudaError_t launch_mc_compat_ieee(const McArgs& a, cudaStream_t s);
-cudaError_t launch_mc_fixed(const McArgs& a, cudaStream_t s);
+cudaError_t launch_mc_compat_ieee(const McArgs& a, int phases, cudaStream_t s);
+cudaError_t launch_mc_fixed(const McArgs& a, int phases, cudaStream_t s);
 cudaError_t launch_weld_fixed(const WeldArgs& a, cudaStream_t s);         // marks edges, numbers vertices
 cudaError_t launch_weld_vertices_fixed(const WeldArgs& a, cudaStream_t s);
 // Batched integrate (one persistent launch over many volumes).

@@ -2534,15 +2534,18 @@ void launch_mc_rowcount(const McArgs& a, cudaStream_t s) {
 }
 
 template <int MODE>
-cudaError_t launch_mc_mode(const McArgs& a, cudaStream_t s) {
+cudaError_t launch_mc_mode(const McArgs& a, int phases, cudaStream_t s) {
     const McGrid& mg = mc_grid<MODE>();
-    if (a.bits_s)
-        launch_mc_bitcount<MODE>(a, s);
-    else
-        launch_mc_rowcount<MODE>(a, s);
-    const unsigned nsuper = (unsigned)((a.ntiles + kMcScanThreads - 1) / kMcScanThreads);
-    mc_reduce_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
-    mc_scan_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
+    if (phases & kMcCount) {
+        if (a.bits_s)
+            launch_mc_bitcount<MODE>(a, s);
+        else
+            launch_mc_rowcount<MODE>(a, s);
+        const unsigned nsuper = (unsigned)((a.ntiles + kMcScanThreads - 1) / kMcScanThreads);
+        mc_reduce_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
+        mc_scan_kernel<<<nsuper, kMcScanThreads, 0, s>>>(a);
+    }
+    if (!(phases & kMcEmit)) return cudaGetLastError();
     const int threads = a.bits_s ? kMcEmitThreads : kMcThreads;
     long long grid = (long long)mg.sms * (a.bits_s ? mg.per_cubes : mg.per_emit);
     const long long tiles_per_cta = threads / 32;   // a warp per listed tile at least

@@ -36,9 +36,11 @@ int integrate_resident_ctas_compat_ieee(int kind, int brick) { return resident_c
 
 int integrate_resident_ctas_fixed(int kind, int brick) { return resident_ctas_mode<kFixed>(kind, brick); }
 
-cudaError_t launch_mc_compat_ieee(const McArgs& a, cudaStream_t s) { return launch_mc_mode<kCompat>(a, s); }
+cudaError_t launch_mc_compat_ieee(const McArgs& a, int phases, cudaStream_t s) {
+    return launch_mc_mode<kCompat>(a, phases, s);
+}
 
-cudaError_t launch_mc_fixed(const McArgs& a, cudaStream_t s) { return launch_mc_mode<kFixed>(a, s); }
+cudaError_t launch_mc_fixed(const McArgs& a, int phases, cudaStream_t s) { return launch_mc_mode<kFixed>(a, phases, s); }
 
 namespace {
 unsigned weld_grid(int64_t n) {

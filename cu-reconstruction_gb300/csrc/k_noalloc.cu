@@ -128,11 +128,11 @@ gbt_status gbt_extract_mesh_noalloc(gbt_volume* v, float* verts, int32_t* tris, 
     e = cudaMemsetAsync(scratch, 0, 64 + nsuper * 16 + (size_t)a.ntiles * 8 + nwords * 4, st);
     if (e == cudaSuccess && a.ntiles > 0) {
         if (gbt::volume_mode(v) == GBT_MODE_FIXED)
-            e = gbt::launch_mc_fixed(a, st);
+            e = gbt::launch_mc_fixed(a, gbt::kMcCount | gbt::kMcEmit, st);
         else if (gbt::volume_arith(v) == GBT_ARITH_IEEE)
-            e = gbt::launch_mc_compat_ieee(a, st);
+            e = gbt::launch_mc_compat_ieee(a, gbt::kMcCount | gbt::kMcEmit, st);
         else
-            e = gbt::launch_mc_compat_ref(a, st);
+            e = gbt::launch_mc_compat_ref(a, gbt::kMcCount | gbt::kMcEmit, st);
     }
     if (e == cudaSuccess) {
         finish_count<<<1, 1, 0, st>>>(s, d_n_tris);

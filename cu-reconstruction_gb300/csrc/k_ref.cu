@@ -24,8 +24,8 @@ int integrate_resident_ctas_compat_ref(int kind, int brick) {
     return refarith::resident_ctas_mode<refarith::kCompat>(kind, brick);
 }
 
-cudaError_t launch_mc_compat_ref(const McArgs& a, cudaStream_t s) {
-    return refarith::launch_mc_mode<refarith::kCompat>(a, s);
+cudaError_t launch_mc_compat_ref(const McArgs& a, int phases, cudaStream_t s) {
+    return refarith::launch_mc_mode<refarith::kCompat>(a, phases, s);
 }
 
 }  // namespace gbt

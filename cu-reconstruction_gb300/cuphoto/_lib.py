@@ -122,6 +122,10 @@ MAX_FRAMES_PER_SCENE_PASS = 128
 DIFF_CHUNK_FRAMES = 8
 POINT_BYTES = 33   # gbt_point, the reference's packed cudaPointCloud::Vertex
 
+# gbt_mesh_alloc: (ctx, n_verts, n_tris, &verts, &normals, &tris) -> 0
+MESH_ALLOC = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_int64, C.c_int64, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
+                         C.POINTER(C.c_void_p))
+
 # (name, restype, argtypes) of every exported entry point, in header order.
 SIGNATURES = [
     ("gbt_volume_create", C.c_int, [C.POINTER(VolumeCfg), C.c_void_p, C.POINTER(C.c_void_p)]),
@@ -150,6 +154,8 @@ SIGNATURES = [
                                          C.c_void_p, C.c_void_p]),
     ("gbt_extract_mesh_indexed", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
                                            C.c_int64, C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.c_void_p]),
+    ("gbt_extract_mesh_sized", C.c_int, [C.c_void_p, C.c_int32, MESH_ALLOC, C.c_void_p, C.c_int64,
+                                         C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.c_void_p]),
     ("gbt_extract_mesh_noalloc", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
                                            C.c_void_p, C.c_void_p]),
     ("gbt_points_extract", C.c_int, [C.POINTER(C.c_double * 9), C.c_void_p, C.c_int64, C.c_int32, C.c_float,

@@ -259,33 +259,52 @@ class TSDFVolume:
                                   depth_scale=depth_scale, stream=stream, **kw)
 
 
+def _extract_sized(volume, shared, normals, index_base, stream):
+    """gbt_extract_mesh_sized into tensors allocated once the mesh is counted:
+    (verts (n_verts, 3), normals or None, tris (n_tris, 3))."""
+    torch = _torch()
+    out = []
+
+    def alloc(ctx, n_verts, n_tris, verts, nrm, tris):
+        try:
+            out.append(torch.empty((n_verts, 3), dtype=torch.float32, device="cuda"))
+            out.append(torch.empty((n_verts, 3), dtype=torch.float32, device="cuda") if normals else None)
+            out.append(torch.empty((n_tris, 3), dtype=torch.int32, device="cuda"))
+            verts[0] = out[0].data_ptr()
+            if normals:
+                nrm[0] = out[1].data_ptr()
+            tris[0] = out[2].data_ptr()
+            return 0
+        except BaseException as e:   # (raised below, on the caller's side of the library)
+            out[:] = [e]
+            return 1
+
+    nv, nt = C.c_int64(), C.c_int64()
+    cb = L.MESH_ALLOC(alloc)
+    st = L.lib().gbt_extract_mesh_sized(volume.handle, int(shared), cb, None, int(index_base), C.byref(nv), C.byref(nt),
+                                        _stream_handle(stream))
+    if out and isinstance(out[0], BaseException):
+        raise out[0]
+    L.check(st)
+    return tuple(out)
+
+
 def extract_mesh_indexed(volume, normals=True, index_base=0, stream=None):
     """Fixed-mode mesh with shared vertices (gbt_extract_mesh_indexed):
     (verts (V, 3) f32, normals (V, 3) f32 or None, tris (T, 3) i32) CUDA
     tensors; the triangles are extract_mesh_device's, in the same order."""
-    torch = _torch()
-    lib = L.lib()
-    s = _stream_handle(stream)
-    nv, nt = C.c_int64(), C.c_int64()
-    L.check(lib.gbt_extract_mesh_indexed(volume.handle, None, None, None, 0, 0, index_base, C.byref(nv), C.byref(nt), s))
-    V = torch.empty((max(nv.value, 1), 3), dtype=torch.float32, device="cuda")
-    N = torch.empty((max(nv.value, 1), 3), dtype=torch.float32, device="cuda") if normals else None
-    T = torch.empty((max(nt.value, 1), 3), dtype=torch.int32, device="cuda")
-    L.check(lib.gbt_extract_mesh_indexed(volume.handle, C.c_void_p(V.data_ptr()),
-                                         C.c_void_p(N.data_ptr()) if normals else None, C.c_void_p(T.data_ptr()),
-                                         nv.value, nt.value, index_base, C.byref(nv), C.byref(nt), s))
-    return V[:nv.value], (N[:nv.value] if normals else None), T[:nt.value]
+    return _extract_sized(volume, True, normals, index_base, stream)
 
 
 def extract_mesh_device(volume, capacity=None, index_base=0, stream=None):
     """Runs the engine's marching cubes; returns (verts (T,3,3) f32, tris (T,3) i32) CUDA tensors."""
+    if capacity is None:
+        v, _, t = _extract_sized(volume, False, False, index_base, stream)
+        return v.view(-1, 3, 3), t
     torch = _torch()
     lib = L.lib()
     s = _stream_handle(stream)
     n = C.c_int64()
-    if capacity is None:
-        L.check(lib.gbt_extract_mesh(volume.handle, None, None, 0, index_base, C.byref(n), s))
-        capacity = n.value
     verts = torch.empty((max(capacity, 1), 3, 3), dtype=torch.float32, device="cuda")
     tris = torch.empty((max(capacity, 1), 3), dtype=torch.int32, device="cuda")
     st = lib.gbt_extract_mesh(volume.handle, C.c_void_p(verts.data_ptr()), C.c_void_p(tris.data_ptr()),

@@ -308,6 +308,22 @@ gbt_status gbt_extract_mesh_indexed(gbt_volume* vol, float* verts, float* normal
                                     int64_t cap_tris, int64_t index_base, int64_t* n_verts, int64_t* n_tris,
                                     void* stream);
 
+/* A mesh into buffers of its size, in one call: the triangles (and vertices)
+ * are counted, `alloc` is called once on this thread with the counts and
+ * provides the buffers, and the mesh is written into them.  What
+ * gbt_extract_mesh (shared_vertices 0: *n_verts = 3 * *n_tris, normals not
+ * asked for) or gbt_extract_mesh_indexed (shared_vertices 1) writes, without
+ * counting a second time as a call for the counts and a call for the mesh do.
+ * alloc(ctx, n_verts, n_tris, &verts, &normals, &tris) sets device pointers for
+ * 3 * n_verts floats, 3 * n_verts floats (left NULL: no normals) and 3 * n_tris
+ * ints and returns 0; anything else ends the call with GBT_ERR_ALLOC.  It may
+ * not use the volume.  Pointers are not needed for 0 triangles.  Index and mode
+ * rules as in those two calls, checked before alloc.  Synchronises `stream`. */
+typedef int (*gbt_mesh_alloc)(void* ctx, int64_t n_verts, int64_t n_tris, float** verts, float** normals,
+                              int32_t** tris);
+gbt_status gbt_extract_mesh_sized(gbt_volume* vol, int32_t shared_vertices, gbt_mesh_alloc alloc, void* ctx,
+                                  int64_t index_base, int64_t* n_verts, int64_t* n_tris, void* stream);
+
 /* Mesh extraction for callers that cannot allocate device memory.
  *
  * No counterpart in the reference: it is an engine addition.  It is meant for

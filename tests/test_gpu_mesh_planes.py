@@ -63,3 +63,37 @@ def test_compat_mesh(gpu, oracle, grid, kind):
     Vo, To = oracle.mc_compat(oracle.cfg_from(tc), D.ravel())
     assert len(V) == len(Vo) and np.array_equal(T, To)
     assert np.array_equal(V.view(np.uint32), Vo.view(np.uint32))
+
+
+def test_sized_extraction_counts_once_and_reports(gpu):
+    """gbt_extract_mesh_sized: the counts given to alloc, a refusing alloc, an
+    index range that does not fit (before alloc), shared vertices in compat."""
+    import ctypes as C
+    from cuphoto import _lib as L
+    lib = L.lib()
+    grid = (40, 36, 32)
+    size = dict(voxel_grid_size=grid, physical_size=tuple(0.01 * g for g in grid))
+    vol = TSDFVolume(TSDFVolumeConfig(mode="fixed", max_weight=16, **size))
+    D, W = field("noise", grid, 5)
+    set_distances(gpu, vol, D, W)
+    V, T = mesh(vol)
+    seen = []
+
+    def refuse(ctx, nv, nt, v, n, t):
+        seen.append((nv, nt))
+        return 1
+
+    cb = L.MESH_ALLOC(refuse)
+    nv, nt = C.c_int64(-1), C.c_int64(-1)
+    args = (cb, None)
+    assert lib.gbt_extract_mesh_sized(vol.handle, 0, *args, 0, C.byref(nv), C.byref(nt), None) == L.GBT_ERR_ALLOC
+    assert seen == [(3 * len(T), len(T))] and (nv.value, nt.value) == (0, 0)
+    assert lib.gbt_extract_mesh_sized(vol.handle, 1, *args, 0, C.byref(nv), C.byref(nt), None) == L.GBT_ERR_ALLOC
+    assert seen[1][1] == len(T) and 0 < seen[1][0] < 3 * len(T)
+    base = 2 ** 31 - 10
+    assert lib.gbt_extract_mesh_sized(vol.handle, 0, *args, base, C.byref(nv), C.byref(nt), None) == L.GBT_ERR_INVALID_ARG
+    compat = TSDFVolume(TSDFVolumeConfig(**size))
+    assert lib.gbt_extract_mesh_sized(compat.handle, 1, *args, 0, C.byref(nv), C.byref(nt), None) == L.GBT_ERR_INVALID_ARG
+    assert len(seen) == 2
+    V2, T2 = mesh(vol)
+    assert np.array_equal(V2.view(np.uint32), V.view(np.uint32)) and np.array_equal(T2, T)
