@@ -94,7 +94,7 @@ struct gbt_volume {
     // the u32 list of tiles with triangles, a u64 offset per tile and the voxels' bit planes
     void* mc_scratch;
     size_t mc_scratch_bytes;
-    // shared-vertex mesh scratch: used-edge bits, word offsets, block sums, vertex count
+    // shared-vertex mesh scratch: words of used edges and first numbers, block sums
     void* weld_scratch;
     size_t weld_scratch_bytes;
     // status word (gbt::kStatus*), in the distances' allocation after the last distance
@@ -1105,9 +1105,12 @@ namespace {
 // Scratch and arguments of the shared-vertex numbering.
 gbt_status weld_prepare(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w) {
     std::memset(w, 0, sizeof(*w));
-    w->nwords = (3 * v->nvox + 31) / 32;
-    w->nblocks = (w->nwords + gbt::kWeldWordsPerBlock - 1) / gbt::kWeldWordsPerBlock;
-    const size_t need = (size_t)w->nwords * 8 + (size_t)w->nblocks * 4;
+    const gbt::VolDesc& d = v->desc;
+    w->nseg = (uint32_t)(d.nx + 31) / 32;
+    w->nwords = w->nseg * (uint32_t)d.ny * (uint32_t)d.nz;   // (no more than voxels)
+    w->nblocks = (uint32_t)(((uint64_t)w->nwords + gbt::kWeldWordsPerBlock - 1) / gbt::kWeldWordsPerBlock);
+    w->div_seg = gbt::make_fastdiv(w->nseg);
+    const size_t need = (size_t)w->nwords * 16 + (size_t)w->nblocks * 4;
     if (v->weld_scratch_bytes < need) {
         if (v->weld_scratch) cudaFree(v->weld_scratch);
         v->weld_scratch = nullptr;
@@ -1120,9 +1123,8 @@ gbt_status weld_prepare(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w) {
         v->weld_scratch_bytes = need;
     }
     w->nverts = &reinterpret_cast<McHeader*>(v->mc_scratch)->nverts;
-    w->bits = static_cast<uint32_t*>(v->weld_scratch);
-    w->word_offset = w->bits + w->nwords;
-    w->block_sums = w->word_offset + w->nwords;
+    w->words = static_cast<uint4*>(v->weld_scratch);
+    w->block_sums = reinterpret_cast<uint32_t*>(w->words + w->nwords);
     w->mc = a;
     return GBT_OK;
 }
@@ -1131,10 +1133,8 @@ gbt_status weld_prepare(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w) {
 gbt_status mc_count(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w, McHeader* hdr, cudaStream_t s) {
     gbt_status st = mc_launch(v, a, s, gbt::kMcCount);
     if (st != GBT_OK) return st;
-    if (w) {
-        cudaError_t e = cudaMemsetAsync(w->bits, 0, (size_t)w->nwords * 4, s);
-        if (e != cudaSuccess) return cuda_fail(e, "vertex-sharing scratch clear");
-        e = gbt::launch_weld_fixed(*w, s);
+    if (w && a.ntiles > 0) {
+        cudaError_t e = gbt::launch_weld_fixed(*w, s);
         if (e != cudaSuccess) return cuda_fail(e, "edge marking");
     }
     return mc_read_header(v, hdr, s);
@@ -1143,15 +1143,15 @@ gbt_status mc_count(gbt_volume* v, const gbt::McArgs& a, gbt::WeldArgs* w, McHea
 // Writes the vertices and normals, and the triangles as their indices.
 gbt_status mc_emit_indexed(gbt_volume* v, gbt::McArgs a, gbt::WeldArgs& w, float* verts, float* normals,
                            int64_t cap_verts, cudaStream_t s) {
-    if (verts && cap_verts > 0) {
+    if (a.ntiles > 0 && ((verts && cap_verts > 0) || a.cap > 0)) {   // (the indices need the numbering)
         w.verts = verts;
         w.normals = normals;
-        w.cap_verts = cap_verts;
+        w.cap_verts = verts ? cap_verts : 0;
         cudaError_t e = gbt::launch_weld_vertices_fixed(w, s);
         if (e != cudaSuccess) return cuda_fail(e, "vertices");
     }
-    a.edge_bits = w.bits;
-    a.edge_word_offset = w.word_offset;
+    a.edge_words = w.words;
+    a.edge_segs = w.nseg;
     return mc_launch(v, a, s, gbt::kMcEmit);
 }
 

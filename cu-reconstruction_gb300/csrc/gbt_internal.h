@@ -201,23 +201,26 @@ struct McArgs {
     uint32_t* bits_o;            // distance below zero; fixed mode: weight above zero
     uint32_t nbits;
     uint32_t pad1;
-    // Fixed mode with shared vertices: when edge_bits is set, triangles are
-    // written as indices of the vertices of their grid edges (edge
-    // 3 * voxel + axis; vertex index = edge_word_offset[edge / 32] + the set
-    // bits of edge_bits below it) and verts is not written.
-    const uint32_t* edge_bits;
-    const uint32_t* edge_word_offset;
+    // Fixed mode with shared vertices: when edge_words is set, triangles are
+    // written as indices of the vertices of their grid edges and verts is not
+    // written.  Word (z * gy + y) * edge_segs + x / 32 holds the number of the
+    // first vertex on an edge of its 32 voxels and their used edges along x, y
+    // and z (bit x % 32); vertices count voxel by voxel, axes x, y, z.
+    const uint4* edge_words;
+    uint32_t edge_segs;      // words per row
+    uint32_t pad2;
 };
 
 // Fixed-mode mesh with shared vertices (k_ieee.cu): the edges used by the
 // triangles, their vertex numbering and the vertices with normals.
 struct WeldArgs {
     McArgs mc;
-    uint32_t* bits;          // [nwords] used-edge bitmask
-    uint32_t* word_offset;   // [nwords] vertex index of each word's first used edge
-    uint32_t* block_sums;    // [nblocks] used edges per block of kWeldWordsPerBlock words
+    uint4* words;            // [nwords] mc.edge_words; only words with a used edge are written
+    uint32_t* block_sums;    // [nblocks] used edges per block of kWeldWordsPerBlock words, then their offsets
     long long* nverts;       // total out
-    int64_t nwords, nblocks;
+    uint32_t nwords, nblocks;
+    uint32_t nseg, pad0;     // words per row
+    FastDiv div_seg;         // nseg
     float* verts;            // 3 per vertex
     float* normals;          // 3 per vertex, or NULL
     int64_t cap_verts;
@@ -259,7 +262,7 @@ cudaError_t launch_integrate_compat_ieee(const IntegrateArgs& a, int brick, int 
 cudaError_t launch_integrate_fixed(const IntegrateArgs& a, int brick, int grid, cudaStream_t s);
 cudaError_t launch_mc_compat_ieee(const McArgs& a, int phases, cudaStream_t s);
 cudaError_t launch_mc_fixed(const McArgs& a, int phases, cudaStream_t s);
-cudaError_t launch_weld_fixed(const WeldArgs& a, cudaStream_t s);         // marks edges, numbers vertices
+cudaError_t launch_weld_fixed(const WeldArgs& a, cudaStream_t s);         // counts vertices, per block and in all
 cudaError_t launch_weld_vertices_fixed(const WeldArgs& a, cudaStream_t s);
 // Batched integrate (one persistent launch over many volumes).
 cudaError_t launch_batch_compat_ref(const BatchArgs& a, int brick, int grid, cudaStream_t s);

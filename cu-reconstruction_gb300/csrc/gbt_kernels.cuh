@@ -1131,15 +1131,6 @@ __device__ __forceinline__ int64_t corner_index(const McArgs& a, int64_t b0, int
     return (corner_dz(k) ? b1 : b0) + corner_dx(k) + (corner_dy(k) ? a.gx : 0);
 }
 
-// Grid edge of cube (cx, cy, cz) between corners ca (the lower one) and cb:
-// 3 * (linear index of ca's voxel) + the axis along which they differ.
-__device__ __forceinline__ int64_t weld_edge_id(const McArgs& a, uint32_t cx, uint32_t cy, uint32_t cz, int ca, int cb) {
-    const int axis = corner_dx(ca) != corner_dx(cb) ? 0 : (corner_dy(ca) != corner_dy(cb) ? 1 : 2);
-    const int64_t lin = ((int64_t)(cz + corner_dz(ca)) * a.gy + (int64_t)(cy + corner_dy(ca))) * a.gx +
-                        (int64_t)(cx + corner_dx(ca));
-    return 3 * lin + axis;
-}
-
 // Cube classification by warps.  The 32 lanes of a warp take 32 consecutive
 // cubes (linear order).  A lane loads the corners of its cube at x (corners
 // 0, 3, 4 and 7: (y, z), (y, z+1), (y+1, z), (y+1, z+1)) and packs their signs
@@ -1839,16 +1830,22 @@ __device__ __forceinline__ void mc_vertex(const McArgs& a, uint32_t cx, uint32_t
     }
 }
 
-// Shared-vertex index of the fixed-mode edge (ca, cb) of cube (cx, cy, cz).
+// Shared-vertex index of the fixed-mode edge (ca, cb) of cube (cx, cy, cz): the
+// edge of its lower corner's voxel along the axis on which the corners differ.
 __device__ __forceinline__ int32_t mc_vertex_index(const McArgs& a, uint32_t cx, uint32_t cy, uint32_t cz, int ca,
                                                    int cb) {
     if (corner_dx(ca) + corner_dy(ca) + corner_dz(ca) > corner_dx(cb) + corner_dy(cb) + corner_dz(cb)) {
         const int tc = ca; ca = cb; cb = tc;
     }
-    const int64_t id = weld_edge_id(a, cx, cy, cz, ca, cb);
-    const uint32_t word = a.edge_bits[id >> 5];
-    const uint32_t below = word & ((1u << (id & 31)) - 1u);
-    return (int32_t)(a.index_base + a.edge_word_offset[id >> 5] + __popc(below));
+    const int axis = corner_dx(ca) != corner_dx(cb) ? 0 : (corner_dy(ca) != corner_dy(cb) ? 1 : 2);
+    const uint32_t x = cx + (uint32_t)corner_dx(ca);
+    const uint32_t row = (cz + (uint32_t)corner_dz(ca)) * (uint32_t)a.gy + cy + (uint32_t)corner_dy(ca);
+    const uint4 e = __ldg(a.edge_words + (size_t)row * a.edge_segs + (x >> 5));
+    const uint32_t j = x & 31u, low = (1u << j) - 1u;
+    uint32_t n = e.x + (uint32_t)(__popc(e.y & low) + __popc(e.z & low) + __popc(e.w & low));
+    if (axis > 0) n += e.y >> j & 1u;
+    if (axis > 1) n += e.z >> j & 1u;
+    return (int32_t)(a.index_base + n);
 }
 
 // A warp's rings of queued cubes and triangles, and their output.
@@ -1977,9 +1974,8 @@ __global__ void __launch_bounds__(kMcThreads) mc_emit_kernel(const __grid_consta
     const unsigned njobs = *a.nonempty;
     constexpr uint32_t kWords = (uint32_t)mc_tile_cubes(MODE) / 1024u;   // group words per tile
     const uint32_t nwords = (a.ncubes + 1023u) / 1024u;
-    const bool indexed = MODE == kFixed && a.edge_bits != nullptr;
     McEmitRings<MODE> R{a, s_cval[warp], s_cube[warp], s_ctype[warp], s_tq[warp], s_out[warp], s_count, s_tri,
-                        s_ends, lane, indexed, 0u, 0u, 0u, 0ll};
+                        s_ends, lane, false, 0u, 0u, 0u, 0ll};
 
     for (;;) {
         unsigned job = 0;
@@ -2069,7 +2065,7 @@ __global__ void __launch_bounds__(kMcEmitThreads) mc_emit_cubes_kernel(const __g
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t kTileWords = (uint32_t)mc_tile_cubes(MODE) / 32u;   // of 32 cubes
     const uint32_t nwords = (a.ncubes + 31u) / 32u;
-    const bool indexed = MODE == kFixed && a.edge_bits != nullptr;
+    const bool indexed = MODE == kFixed && a.edge_words != nullptr;
     McEmitRings<MODE> R{a, s_cval[warp], s_cube[warp], s_ctype[warp], s_tq[warp], s_out[warp], s_count, s_tri,
                         s_ends, lane, indexed, 0u, 0u, 0u, 0ll};
     unsigned short* list = s_list[warp];
@@ -2165,70 +2161,77 @@ __global__ void __launch_bounds__(kMcEmitThreads) mc_emit_cubes_kernel(const __g
 
 #if !defined(GBT_REF_ARITH)
 // ---------------------------------------------------------------------------
-// Fixed-mode mesh with shared vertices.  (1) weld_mark: every cube that the
-// fixed-mode marching cubes emits sets the bits of the grid edges its
-// triangles use; (2) weld_count / weld_scan_blocks / weld_offsets: an
-// exclusive scan of the bit counts numbers the used edges (vertex index =
-// word offset + set bits below); (3) weld_vertices: one vertex per used
-// edge, interpolated exactly as mc_emit_kernel<kFixed> interpolates it (lower
-// endpoint first, so the positions are the ones the triangle soup holds),
-// with the normal of the interpolated central-difference gradient;
-// (4) mc_emit_kernel<kFixed> with edge_bits set writes the triangles as indices,
-// in the same order as the triangle soup.
-__global__ void __launch_bounds__(256) weld_mark_kernel(const __grid_constant__ McArgs a, uint32_t* bits) {
-    __shared__ unsigned char s_count[256];
-    __shared__ unsigned long long s_tri[256];
-    __shared__ unsigned char s_ends[12];
-    __shared__ unsigned char s_type[256];
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) {
-        s_count[k] = GBT_MC_TRI_COUNT[k];
-        s_tri[k] = GBT_MC_TRI_PACKED[k];
-        s_type[k] = (unsigned char)mc_type_of_nibbles(k & 15, k >> 4);
-    }
-    if (threadIdx.x < 12) s_ends[threadIdx.x] = GBT_MC_EDGE_ENDS[threadIdx.x];
-    __syncthreads();
-    // whole warps take 32 consecutive cubes (the classification shuffles)
-    const int lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t w0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < a.ncubes; w0 += stride) {
-        const bool valid = w0 + lane < a.ncubes;
-        const uint32_t c = valid ? (uint32_t)(w0 + lane) : a.ncubes - 1;
-        uint32_t idx[4];
-        const bool own = cube_xcorners<kFixed>(a, c, idx) || lane == 31;
-        int sx = 0, so = 0;
-        bool okx = true, oko = true;
+// Fixed-mode mesh with shared vertices, from the bit planes of the count.  A
+// grid edge is used if its ends differ in sign and one of the four cubes around
+// it has all its corners observed (such a cube then has triangles on the edge).
+// With 32 voxels of a row as words that is a few ANDs and ORs, so the used edges
+// are found twice rather than stored: (1) weld_count sums them per block of
+// rows' words, weld_scan_blocks turns the sums into offsets; (2) weld_vertices
+// finds them again, numbers them (voxels in linear order, axes x, y, z within
+// one), writes the words and first numbers for the emission's look-ups, and one
+// vertex per used edge, interpolated exactly as mc_vertex<kFixed> interpolates
+// it (lower endpoint first, so the positions are the ones the triangle soup
+// holds), with the normal of the interpolated central-difference gradient;
+// (3) mc_emit_cubes_kernel<kFixed> with edge_words set writes the triangles as
+// indices, in the same order as the triangle soup.  At 384^3 (268 K vertices):
+// @@FIG@@
+struct WeldWord {
+    uint32_t x, y, z;   // bit j: the edge of voxel x0 + j along the axis is used
+    __device__ __forceinline__ int count() const { return __popc(x) + __popc(y) + __popc(z); }
+};
+
+// The used edges of the 32 voxels of word `word` (row (y, z), columns x0 ...).
+__device__ __forceinline__ WeldWord weld_word(const WeldArgs& w, uint32_t word) {
+    const McArgs& a = w.mc;
+    const uint32_t gx = (uint32_t)a.gx, gy = (uint32_t)a.gy, gz = (uint32_t)a.gz;
+    const uint32_t row = fastdiv(word, w.div_seg);
+    const uint32_t x0 = (word - row * w.nseg) * 32u;
+    const uint32_t z = fastdiv(row, a.div_gy), y = row - z * gy;
+    const uint32_t b = row * gx + x0, layer = gx * gy;
+    const uint32_t in = gx - x0 >= 32u ? ~0u : (1u << (gx - x0)) - 1u;               // x < gx
+    const uint32_t inx = gx - 1u - x0 >= 32u ? ~0u : (1u << (gx - 1u - x0)) - 1u;    // x < gx - 1
+    const bool yok = y + 1u < gy, zok = z + 1u < gz;
+    uint32_t p, q, py = 0u, pz = 0u, unused;
+    mc_bits33(a.bits_s, b, p, q);
+    if (yok) mc_bits33(a.bits_s, b + gx, py, unused);
+    if (zok) mc_bits33(a.bits_s, b + layer, pz, unused);
+    WeldWord u;
+    u.x = (p ^ q) & inx;
+    u.y = yok ? (p ^ py) & in : 0u;
+    u.z = zok ? (p ^ pz) & in : 0u;
+    if (!(u.x | u.y | u.z)) return u;
+    // Columns observed in the voxel rows (y - 1 + dy, z - 1 + dz): x - 1, x and
+    // x + 1 (a column before the row's first or after its last stands for no
+    // cube below, whatever its bit; rows outside the grid are unobserved)
+    uint32_t oP[3][3], oM[3][3], oN[3][3];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            sx |= (__ldg(a.D + idx[k]) < 0.f) << k;
-            okx = okx && __ldg(a.W + idx[k]) > 0.f;
-            if (own) {
-                so |= (__ldg(a.D + idx[k] + 1) < 0.f) << k;
-                oko = oko && __ldg(a.W + idx[k] + 1) > 0.f;
+    for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            const bool have = (dy == 0 ? y > 0u : dy == 1 || yok) && (dz == 0 ? z > 0u : dz == 1 || zok);
+            oP[dy][dz] = oM[dy][dz] = oN[dy][dz] = 0u;
+            if (have) {
+                const uint32_t r = b + (uint32_t)(dy - 1) * gx + (uint32_t)(dz - 1) * layer;
+                mc_bits33(a.bits_o, r, oM[dy][dz], oN[dy][dz]);
+                oP[dy][dz] = oM[dy][dz] << 1;
+                if (x0) oP[dy][dz] |= __ldg(a.bits_o + ((r - 1u) >> 5)) >> ((r - 1u) & 31u) & 1u;
             }
         }
-        sx |= okx << 4;
-        so |= oko << 4;
-        // every lane takes part in the shuffle; a lane then keeps its own loads or the next lane's
-        const int nx = __shfl_down_sync(0xffffffffu, sx, 1);
-        const int sn = own ? so : nx;
-        if (!valid || !(sx & sn & 16)) continue;
-        const int t = s_type[(sx & 15) | (sn & 15) << 4];
-        const uint32_t row = fastdiv(c, a.div_cx);
-        const uint32_t cx = c - row * (uint32_t)(a.gx - 1);
-        const uint32_t cz = fastdiv(row, a.div_cy);
-        const uint32_t cy = row - cz * (uint32_t)(a.gy - 1);
-        const int n = s_count[t];
-        const unsigned long long edges = s_tri[t];
-        for (int q = 0; q < 3 * n; ++q) {
-            const int e = (int)((edges >> (4 * q)) & 15ull);
-            int ca = s_ends[e] & 15, cb = s_ends[e] >> 4;
-            if (corner_dx(ca) + corner_dy(ca) + corner_dz(ca) > corner_dx(cb) + corner_dy(cb) + corner_dz(cb)) {
-                const int tc = ca; ca = cb; cb = tc;
-            }
-            const int64_t id = weld_edge_id(a, cx, cy, cz, ca, cb);
-            atomicOr(bits + (id >> 5), 1u << (id & 31));
+    // cubes (x, y - 1 + cy, z - 1 + cz), and those at x - 1, with all corners observed
+    uint32_t c[2][2], cm[2][2];
+#pragma unroll
+    for (int cz = 0; cz < 2; ++cz)
+#pragma unroll
+        for (int cy = 0; cy < 2; ++cy) {
+            const uint32_t m = oM[cy][cz] & oM[cy + 1][cz] & oM[cy][cz + 1] & oM[cy + 1][cz + 1];
+            c[cy][cz] = m & oN[cy][cz] & oN[cy + 1][cz] & oN[cy][cz + 1] & oN[cy + 1][cz + 1] & inx;
+            cm[cy][cz] = m & oP[cy][cz] & oP[cy + 1][cz] & oP[cy][cz + 1] & oP[cy + 1][cz + 1];
+            if (x0 == 0u) cm[cy][cz] &= ~1u;
         }
-    }
+    u.x &= c[0][0] | c[0][1] | c[1][0] | c[1][1];
+    u.y &= c[1][0] | c[1][1] | cm[1][0] | cm[1][1];
+    u.z &= c[0][1] | c[1][1] | cm[0][1] | cm[1][1];
+    return u;
 }
 
 __device__ __forceinline__ uint32_t block_sum_256(uint32_t v, uint32_t* s_warp) {
@@ -2240,16 +2243,16 @@ __device__ __forceinline__ uint32_t block_sum_256(uint32_t v, uint32_t* s_warp) 
     return t;
 }
 
-// used edges per block of kWeldWordsPerBlock words (256 threads x 4 words)
-__global__ void __launch_bounds__(256) weld_count_kernel(const uint32_t* bits, int64_t nwords, uint32_t* block_sums) {
+// used edges per block of kWeldWordsPerBlock words
+__global__ void __launch_bounds__(256) weld_count_kernel(const __grid_constant__ WeldArgs w) {
     __shared__ uint32_t s_warp[8];
-    const int64_t base = (int64_t)blockIdx.x * kWeldWordsPerBlock + 4 * threadIdx.x;
+    const uint32_t base = blockIdx.x * (uint32_t)kWeldWordsPerBlock + threadIdx.x;
     uint32_t v = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (base + k < nwords) v += __popc(bits[base + k]);
+#pragma unroll 1
+    for (uint32_t k = 0; k < (uint32_t)kWeldWordsPerBlock; k += 256u)
+        if (base + k < w.nwords) v += (uint32_t)weld_word(w, base + k).count();
     const uint32_t t = block_sum_256(v, s_warp);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = t;
+    if (threadIdx.x == 0) w.block_sums[blockIdx.x] = t;
 }
 
 // exclusive scan of the block sums in place, one CTA of 1024 threads
@@ -2288,35 +2291,6 @@ __global__ void __launch_bounds__(1024) weld_scan_blocks_kernel(uint32_t* block_
     if (threadIdx.x == 0) *nverts = (long long)s_carry;
 }
 
-// vertex index of each word's first used edge
-__global__ void __launch_bounds__(256) weld_offsets_kernel(const uint32_t* bits, int64_t nwords,
-                                                           const uint32_t* block_offsets, uint32_t* word_offset) {
-    __shared__ uint32_t s_warp[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * kWeldWordsPerBlock + 4 * threadIdx.x;
-    uint32_t c[4];
-    uint32_t v = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        c[k] = base + k < nwords ? (uint32_t)__popc(bits[base + k]) : 0u;
-        v += c[k];
-    }
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    uint32_t before = block_offsets[blockIdx.x] + x - v;
-    for (int w = 0; w < warp; ++w) before += s_warp[w];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (base + k < nwords) word_offset[base + k] = before;
-        before += c[k];
-    }
-}
-
 __device__ __forceinline__ void weld_gradient(const McArgs& a, int x, int y, int z, float* g) {
     const int n[3] = {a.gx, a.gy, a.gz};
     const int p[3] = {x, y, z};
@@ -2330,48 +2304,95 @@ __device__ __forceinline__ void weld_gradient(const McArgs& a, int x, int y, int
     }
 }
 
+// One CTA per block of kWeldWordsPerBlock words, 256 words at a time; a warp's
+// vertices are then dealt to its lanes 32 at a time, whichever words they are in.
 __global__ void __launch_bounds__(256) weld_vertices_kernel(const __grid_constant__ WeldArgs w) {
     const McArgs& a = w.mc;
-    for (int64_t word = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; word < w.nwords;
-         word += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t m = w.bits[word];
-        int64_t vid = w.word_offset[word];
-        while (m) {
-            const int k = __ffs(m) - 1;
-            m &= m - 1;
-            const int64_t id = word * 32 + k;
-            const int64_t lin = id / 3;
-            const int axis = (int)(id - 3 * lin);
-            const uint32_t row = fastdiv((uint32_t)lin, a.div_gx);
-            const int x = (int)((uint32_t)lin - row * (uint32_t)a.gx);
+    __shared__ uint32_t s_warp[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool last = blockIdx.x + 1u == gridDim.x;
+    uint32_t before = w.block_sums[blockIdx.x];   // vertices before the next 256 words
+    if (!last && before == w.block_sums[blockIdx.x + 1u]) return;   // no used edge in the block
+#pragma unroll 1
+    for (uint32_t k = 0; k < (uint32_t)kWeldWordsPerBlock; k += 256u) {
+        const uint32_t word = blockIdx.x * (uint32_t)kWeldWordsPerBlock + k + threadIdx.x;
+        WeldWord u{0u, 0u, 0u};
+        if (word < w.nwords) u = weld_word(w, word);
+        const uint32_t n = (uint32_t)u.count();
+        uint32_t incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t first = before;   // of the warp
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            const uint32_t t = s_warp[v];
+            if (v < warp) first += t;
+            before += t;
+        }
+        __syncthreads();   // s_warp may be written again
+        const uint32_t excl = incl - n;
+        if (n) w.words[word] = make_uint4(first + excl, u.x, u.y, u.z);
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll 1
+        for (uint32_t t = 0; t < total; t += 32u) {
+            // vertex t + lane of the warp: the last lane whose vertices start at or before it
+            const uint32_t i = min(t + (uint32_t)lane, total - 1u);
+            int own = 0;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1) {
+                const uint32_t e = __shfl_sync(0xffffffffu, excl, own + h);
+                if (e <= i) own += h;
+            }
+            const uint32_t ux = __shfl_sync(0xffffffffu, u.x, own), uy = __shfl_sync(0xffffffffu, u.y, own),
+                           uz = __shfl_sync(0xffffffffu, u.z, own);
+            uint32_t r = i - __shfl_sync(0xffffffffu, excl, own);   // its rank in that word
+            // the last voxel with at most r edges before it
+            int j = 0;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1) {
+                const uint32_t low = (1u << (j + h)) - 1u;
+                if ((uint32_t)(__popc(ux & low) + __popc(uy & low) + __popc(uz & low)) <= r) j += h;
+            }
+            const uint32_t low = (1u << j) - 1u;
+            r -= (uint32_t)(__popc(ux & low) + __popc(uy & low) + __popc(uz & low));
+            const uint32_t bx = ux >> j & 1u, by = uy >> j & 1u;
+            const int axis = r < bx ? 0 : r < bx + by ? 1 : 2;
+            const int64_t vid = (int64_t)first + i;
+            if (t + (uint32_t)lane >= total || vid >= w.cap_verts) continue;
+            const uint32_t wd = word - (uint32_t)lane + (uint32_t)own;
+            const uint32_t row = fastdiv(wd, w.div_seg);
+            const int x = (int)((wd - row * w.nseg) * 32u) + j;
             const uint32_t zz = fastdiv(row, a.div_gy);
             const int y = (int)(row - zz * (uint32_t)a.gy), z = (int)zz;
+            const int64_t lin = (int64_t)row * a.gx + x;
             const int x1 = x + (axis == 0), y1 = y + (axis == 1), z1 = z + (axis == 2);
             const int64_t lin1 = ((int64_t)z1 * a.gy + y1) * a.gx + x1;
             const float sa = a.D[lin], sb = a.D[lin1];
             const float pa[3] = {centre(x, a.vs[0], a.off[0]), centre(y, a.vs[1], a.off[1]), centre(z, a.vs[2], a.off[2])};
             const float pb[3] = {centre(x1, a.vs[0], a.off[0]), centre(y1, a.vs[1], a.off[1]),
                                  centre(z1, a.vs[2], a.off[2])};
-            const float r = __fdiv_rn(sa, __fsub_rn(sa, sb));
-            if (vid < w.cap_verts) {
+            const float ratio = __fdiv_rn(sa, __fsub_rn(sa, sb));
 #pragma unroll
-                for (int q = 0; q < 3; ++q) w.verts[3 * vid + q] = __fmaf_rn(r, __fsub_rn(pb[q], pa[q]), pa[q]);
-                if (w.normals) {
-                    float ga[3], gb[3], nrm[3];
-                    weld_gradient(a, x, y, z, ga);
-                    weld_gradient(a, x1, y1, z1, gb);
-                    float ss = 0.f;
+            for (int q = 0; q < 3; ++q) w.verts[3 * vid + q] = __fmaf_rn(ratio, __fsub_rn(pb[q], pa[q]), pa[q]);
+            if (w.normals) {
+                float ga[3], gb[3], nrm[3];
+                weld_gradient(a, x, y, z, ga);
+                weld_gradient(a, x1, y1, z1, gb);
+                float ss = 0.f;
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        nrm[q] = ga[q] + r * (gb[q] - ga[q]);
-                        ss += nrm[q] * nrm[q];
-                    }
-                    const float inv = ss > 0.f ? rsqrtf(ss) : 0.f;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) w.normals[3 * vid + q] = nrm[q] * inv;
+                for (int q = 0; q < 3; ++q) {
+                    nrm[q] = ga[q] + ratio * (gb[q] - ga[q]);
+                    ss += nrm[q] * nrm[q];
                 }
+                const float inv = ss > 0.f ? rsqrtf(ss) : 0.f;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) w.normals[3 * vid + q] = nrm[q] * inv;
             }
-            ++vid;
         }
     }
 }

@@ -42,30 +42,14 @@ cudaError_t launch_mc_compat_ieee(const McArgs& a, int phases, cudaStream_t s) {
 
 cudaError_t launch_mc_fixed(const McArgs& a, int phases, cudaStream_t s) { return launch_mc_mode<kFixed>(a, phases, s); }
 
-namespace {
-unsigned weld_grid(int64_t n) {
-    static const int sms = [] {
-        int dev = 0, m = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
-        return m > 0 ? m : 1;
-    }();
-    const int64_t want = (n + 255) / 256;
-    const int64_t cap = (int64_t)sms * 16;
-    return (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-}
-}  // namespace
-
 cudaError_t launch_weld_fixed(const WeldArgs& w, cudaStream_t s) {
-    ieeearith::weld_mark_kernel<<<weld_grid(w.mc.ncubes), 256, 0, s>>>(w.mc, w.bits);
-    ieeearith::weld_count_kernel<<<(unsigned)w.nblocks, 256, 0, s>>>(w.bits, w.nwords, w.block_sums);
+    ieeearith::weld_count_kernel<<<w.nblocks, 256, 0, s>>>(w);
     ieeearith::weld_scan_blocks_kernel<<<1, 1024, 0, s>>>(w.block_sums, w.nblocks, w.nverts);
-    ieeearith::weld_offsets_kernel<<<(unsigned)w.nblocks, 256, 0, s>>>(w.bits, w.nwords, w.block_sums, w.word_offset);
     return cudaGetLastError();
 }
 
 cudaError_t launch_weld_vertices_fixed(const WeldArgs& w, cudaStream_t s) {
-    ieeearith::weld_vertices_kernel<<<weld_grid(w.nwords), 256, 0, s>>>(w);
+    ieeearith::weld_vertices_kernel<<<w.nblocks, 256, 0, s>>>(w);
     return cudaGetLastError();
 }
 
