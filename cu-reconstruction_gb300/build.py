@@ -28,6 +28,7 @@ UNITS = {
     "k_noalloc.cu": [],
     "k_diff.cu": [],
     "k_points.cu": [],
+    "k_depth.cu": [],
 }
 
 

@@ -88,12 +88,35 @@ inline FastDiv make_fastdiv(uint32_t d) {
     return f;
 }
 
+// Depth pyramids of the frames of a call (k_depth.cu): per frame, the largest
+// usable depth (above 0, at most the cap the pyramid was built with; 0: none) of
+// tiles of 8 x 8 pixels, then of 16 x 16, ... 128 x 128, each level's tiles row
+// by row.  base NULL: no pyramids.
+constexpr int kPyrLevels = 5;
+struct DepthPyr {
+    const float* base;
+    uint32_t stride;   // floats per frame
+    uint32_t pad0;
+    __host__ __device__ const float* of(int frame) const { return base ? base + (size_t)frame * stride : nullptr; }
+};
+inline uint32_t pyr_floats(int32_t width, int32_t height) {
+    uint64_t n = 0;
+    uint32_t w = ((uint32_t)width + 7u) >> 3, h = ((uint32_t)height + 7u) >> 3;
+    for (int l = 0; l < kPyrLevels; ++l) {
+        n += (uint64_t)w * h;
+        w = (w + 1u) >> 1;
+        h = (h + 1u) >> 1;
+    }
+    return n > 0xffffffffull ? 0u : (uint32_t)n;   // (an image of more than 2^37 pixels: none)
+}
+
 struct IntegrateArgs {
     VolDesc vol;
     int32_t nframes;
     uint32_t nbricks;        // bricks of the volume for the launch's brick shape
     FastDiv div_nbx;         // bricks along x
     FastDiv div_nby;         // bricks along y
+    DepthPyr pyr;            // of the pass's frames
     unsigned int* status;    // streamed pass: the volume's status word (kStatusWaitExpired)
     int32_t hold_first_copy; // streamed pass, failure injection: CTA 0 issues no copy for its first brick
     int32_t pad1;
@@ -137,6 +160,7 @@ struct BatchArgs {
     int32_t w0, wn;         // frame window
     int32_t rows_of_4;      // 1: every scene's x extent is a multiple of 4
     long long total_bricks; // bricks of those scenes
+    DepthPyr pyr;           // of the frame table's frames
     unsigned int* ticket;   // this launch's ticket, zero at launch
 };
 
@@ -282,6 +306,12 @@ cudaError_t launch_batch_fixed(const BatchArgs& a, int brick, int grid, cudaStre
 cudaError_t launch_stream_compat_ref(const IntegrateArgs& a, const VolumeMaps& m, int grid, cudaStream_t s);
 cudaError_t launch_stream_compat_ieee(const IntegrateArgs& a, const VolumeMaps& m, int grid, cudaStream_t s);
 cudaError_t launch_stream_fixed(const IntegrateArgs& a, const VolumeMaps& m, int grid, cudaStream_t s);
+// k_depth.cu: the depth pyramids of frames [0, n) of a table in device memory, or
+// of a pass's (by value).
+cudaError_t launch_depth_pyramids(const FrameDesc* frames, int n, int32_t max_width, int32_t max_height, float cap,
+                                  const DepthPyr& pyr, cudaStream_t s);
+cudaError_t launch_depth_pyramids(const IntegrateArgs& a, int32_t max_width, int32_t max_height, float cap,
+                                  cudaStream_t s);
 // k_util.cu: volume initialisation and the packed per-voxel transform records.
 cudaError_t launch_volume_init(float* D, float* W, int64_t n, float trunc, cudaStream_t s);
 cudaError_t launch_tvoxels(void* out, const VolDesc& v, cudaStream_t s);
