@@ -91,30 +91,30 @@ namespace {
 // (they add up to less than the last one, which is at least twice as large as
 // the one before).
 struct PyrBuffer {
-    float* data;
-    size_t floats;
+    float2* data;
+    size_t tiles;
     void* own[32];   // allocations, the last of them data's
     int nown;
 };
 
-// Room for n floats, or NULL: the caller then goes without pyramids (an
+// Room for n tiles, or NULL: the caller then goes without pyramids (an
 // allocation failed, or would be needed while `s` is being captured).
-float* pyr_room(PyrBuffer* b, size_t n, cudaStream_t s) {
-    if (b->floats >= n) return b->data;
+float2* pyr_room(PyrBuffer* b, size_t n, cudaStream_t s) {
+    if (b->tiles >= n) return b->data;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone || b->nown >= 32) {
         cudaGetLastError();
         return nullptr;
     }
-    const size_t want = std::max(n, 2 * b->floats);
+    const size_t want = std::max(n, 2 * b->tiles);
     void* p = nullptr;
-    if (cudaMalloc(&p, want * sizeof(float)) != cudaSuccess) {
+    if (cudaMalloc(&p, want * sizeof(float2)) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
     b->own[b->nown++] = p;
-    b->data = static_cast<float*>(p);
-    b->floats = want;
+    b->data = static_cast<float2*>(p);
+    b->tiles = want;
     return b->data;
 }
 
@@ -157,10 +157,10 @@ void set_last_error(const char* msg) { g_last_error = msg; }
 // (one wave of the persistent grid), cached per kernel.
 int integrate_default_ctas_per_sm(int mode, int arith, int kind, int brick) {
     // host threads may race to fill an entry: each computes the same value
-    static std::atomic<int> cache[3][5][4] = {};   // [arithmetic][kind 0..4][brick shape]
+    static std::atomic<int> cache[3][6][4] = {};   // [arithmetic][kind 0..5][brick shape]
     const int k = mode == GBT_MODE_FIXED ? 2 : (arith == GBT_ARITH_IEEE ? 1 : 0);
     const int b = brick >= 0 && brick < 4 ? brick : 0;
-    if (kind < 0 || kind > 4) kind = 0;
+    if (kind < 0 || kind > 5) kind = 0;
     std::atomic<int>& slot = cache[k][kind][b];
     int n = slot.load(std::memory_order_relaxed);
     if (n == 0) {
@@ -215,8 +215,20 @@ void fixed_projection(const double* pose, const gbt_volume_cfg& c, float* P) {
     P[11] = (float)t[2];
 }
 
-// The largest depth that integrating into the volume uses.
-float usable_depth_cap(const gbt_volume* v) { return v->cfg.mode == GBT_MODE_FIXED ? v->desc.max_depth : 24.0f; }
+// Whether a pass of n frames (at most kLaneBrickFrames; longer ones always do)
+// gives a thread 4 voxels along z rather than along x (BrickLayout in
+// gbt_kernels.cuh).  Along x the voxels move as 16-byte vectors if rows start on
+// 16 bytes; along z a frame costs fewer instructions.  Measured along x / z, us
+// a frame: reference arithmetic, 256^3: 25.0 / 31.0 for one frame, 14.9 / 15.9
+// for 4, 384^3: 50.7 / 49.8 for 6, 46.4 / 44.0 for 8; IEEE arithmetic (its divides
+// leave the passes bound by instructions), 384^3: 141 / 136 for one frame, 110 /
+// 97 for 2, fixed mode 82.3 / 82.8 and 63.6 / 61.1; rows of 383 voxels, fixed: 103
+// / 89 for one, of 382, reference: 158 / 140.
+bool layer_runs_pay(const gbt_volume* v, int32_t n) {
+    if (v->desc.nx % 4 != 0) return true;
+    const bool reference = v->cfg.mode == GBT_MODE_COMPAT && v->cfg.arith == GBT_ARITH_REFERENCE;
+    return n >= (reference ? 6 : 2);
+}
 
 // Whether depth pyramids pay for `voxel_frames` voxel-frames of work over
 // frames of `pixels` each, `frames` of them: building them is a launch of its
@@ -404,8 +416,8 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
     // pyramids of one pass of frames of the configured camera
     const size_t status_at = (bytes + 255) / 256 * 256;
     if (c.camera_width > 0 && c.camera_height > 0 && c.camera_width <= 4096 && c.camera_height <= 4096)
-        v->pyr.floats = (size_t)gbt::pyr_floats(c.camera_width, c.camera_height) * GBT_MAX_FRAMES_PER_PASS;
-    const size_t d_bytes = status_at + 256 + v->pyr.floats * sizeof(float);
+        v->pyr.tiles = (size_t)gbt::pyr_tiles(c.camera_width, c.camera_height) * GBT_MAX_FRAMES_PER_PASS;
+    const size_t d_bytes = status_at + 256 + v->pyr.tiles * sizeof(float2);
     cudaError_t e;
     if (v->managed) {
         e = dev_alloc(reinterpret_cast<void**>(&d.D), d_bytes, true);
@@ -416,7 +428,7 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
     }
     if (e == cudaSuccess) {
         v->status = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(d.D) + status_at);
-        v->pyr.data = reinterpret_cast<float*>(reinterpret_cast<char*>(d.D) + status_at + 256);
+        v->pyr.data = reinterpret_cast<float2*>(reinterpret_cast<char*>(d.D) + status_at + 256);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -678,7 +690,12 @@ gbt_status gbt_integrate_tuned(gbt_volume* v, const gbt_frame* frames, int32_t n
     a.div_nbx = gbt::make_fastdiv(nbx);
     a.div_nby = gbt::make_fastdiv(nby);
     a.status = v->status;
-    const int kind = brick == 8 ? 4 : (brick >= 4 ? 3 : (nframes <= gbt::kLaneBrickFrames ? 1 : 0));
+    a.layer_runs = layer_runs_pay(v, nframes) ? 1 : 0;
+    const int kind = brick == 8                         ? 4
+                     : brick >= 4                       ? 3
+                     : nframes > gbt::kLaneBrickFrames ? 0
+                     : a.layer_runs                     ? 5
+                                                        : 1;
     long long grid = (long long)device_sms() *
                      (ctas_per_sm ? ctas_per_sm
                                   : gbt::integrate_default_ctas_per_sm(v->cfg.mode, v->cfg.arith, kind, brick & 3));
@@ -692,12 +709,12 @@ gbt_status gbt_integrate_tuned(gbt_volume* v, const gbt_frame* frames, int32_t n
             mw = std::max(mw, frames[i].width);
             mh = std::max(mh, frames[i].height);
         }
-        const uint32_t stride = gbt::pyr_floats(mw, mh);
+        const uint32_t stride = gbt::pyr_tiles(mw, mh);
         if (stride && pyramids_pay(v->nvox * nframes, nframes, (int64_t)mw * mh))
             a.pyr.base = pyr_room(&v->pyr, (size_t)stride * (size_t)nframes, as_stream(stream));
         if (a.pyr.base) {
             a.pyr.stride = stride;
-            e = gbt::launch_depth_pyramids(a, mw, mh, usable_depth_cap(v), as_stream(stream));
+            e = gbt::launch_depth_pyramids(a, mw, mh, as_stream(stream));
             if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
         }
     }
@@ -913,12 +930,12 @@ gbt_status gbt_batch_create(int32_t max_scenes, int32_t max_frames, gbt_batch** 
     b->max_scenes = max_scenes;
     b->max_frames = max_frames;
     b->bytes = batch_bytes(max_scenes, max_frames);
-    // the device tables are followed by the depth pyramids of up to 1024 frames of 640x480 (26 MB)
+    // the device tables are followed by the depth pyramids of up to 1024 frames of 640x480 (52 MB)
     const size_t pyr_at = (b->bytes + 255) / 256 * 256;
-    b->pyr.floats = (size_t)gbt::pyr_floats(640, 480) * (size_t)std::min(max_frames, 1024);
+    b->pyr.tiles = (size_t)gbt::pyr_tiles(640, 480) * (size_t)std::min(max_frames, 1024);
     cudaError_t e = pinned_alloc(&b->host, b->bytes);
-    if (e == cudaSuccess) e = dev_alloc(&b->dev, pyr_at + b->pyr.floats * sizeof(float));
-    if (e == cudaSuccess) b->pyr.data = reinterpret_cast<float*>(static_cast<char*>(b->dev) + pyr_at);
+    if (e == cudaSuccess) e = dev_alloc(&b->dev, pyr_at + b->pyr.tiles * sizeof(float2));
+    if (e == cudaSuccess) b->pyr.data = reinterpret_cast<float2*>(static_cast<char*>(b->dev) + pyr_at);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -1054,23 +1071,19 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
     {
         int32_t mw = 0, mh = 0;
         uint32_t stride = 0;
-        float cap = 0.f;
         for (int i = 0; i < nframes; ++i) {
             mw = std::max(mw, frames[i].width);
             mh = std::max(mh, frames[i].height);
         }
         int64_t work = 0;
-        for (int i = 0; i < nitems; ++i) {
-            cap = std::max(cap, usable_depth_cap(items[i].volume));
-            work += items[i].volume->nvox * items[i].nframes;   // (below 2^32 * 2^24)
-        }
-        stride = gbt::pyr_floats(mw, mh);
+        for (int i = 0; i < nitems; ++i) work += items[i].volume->nvox * items[i].nframes;   // (below 2^32 * 2^24)
+        stride = gbt::pyr_tiles(mw, mh);
         if (stride && pyramids_pay(work, nframes, (int64_t)mw * mh)) pyr.base = pyr_room(&b->pyr, (size_t)stride * (size_t)nframes, s);
         if (pyr.base) {
             pyr.stride = stride;
             e = gbt::launch_depth_pyramids(
                 reinterpret_cast<const gbt::FrameDesc*>(reinterpret_cast<const gbt::BatchScene*>(d + 256) + b->max_scenes),
-                nframes, mw, mh, cap, pyr, s);
+                nframes, mw, mh, pyr, s);
             if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
         }
     }
@@ -1079,15 +1092,16 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
     for (int w = 0; w < nwin; ++w) {
         gbt::BatchArgs a;
         std::memset(&a, 0, sizeof(a));
+        a.vol = hs[0].vol;
         a.ticket = reinterpret_cast<unsigned int*>(d) + w;
         a.scenes = reinterpret_cast<const gbt::BatchScene*>(d + 256);
         a.frames = reinterpret_cast<const gbt::FrameDesc*>(a.scenes + b->max_scenes);
         a.w0 = w * frames_per_launch;
         a.wn = frames_per_launch;
         a.pyr = pyr;
-        a.rows_of_4 = 1;
+        a.layers_of_4 = 1;
         for (int j = 0; j < nitems; ++j)
-            if (items[j].volume->desc.nx % 4 != 0) a.rows_of_4 = 0;
+            if (items[j].volume->desc.nz % 4 != 0) a.layers_of_4 = 0;
         int m = 0;
         while (m < nitems && hs[m].nframes > a.w0) ++m;
         a.nscenes = m;

@@ -89,17 +89,17 @@ inline FastDiv make_fastdiv(uint32_t d) {
 }
 
 // Depth pyramids of the frames of a call (k_depth.cu): per frame, the largest
-// usable depth (above 0, at most the cap the pyramid was built with; 0: none) of
-// tiles of 8 x 8 pixels, then of 16 x 16, ... 128 x 128, each level's tiles row
-// by row.  base NULL: no pyramids.
+// positive depth (0: none; a NaN counts as infinite) and the least one (3e38:
+// none) of tiles of 8 x 8 pixels, then of 16 x 16, ... 128 x 128, each level's
+// tiles row by row.  base NULL: no pyramids.
 constexpr int kPyrLevels = 5;
 struct DepthPyr {
-    const float* base;
-    uint32_t stride;   // floats per frame
+    const float2* base;
+    uint32_t stride;   // tiles per frame
     uint32_t pad0;
-    __host__ __device__ const float* of(int frame) const { return base ? base + (size_t)frame * stride : nullptr; }
+    __host__ __device__ const float2* of(int frame) const { return base ? base + (size_t)frame * stride : nullptr; }
 };
-inline uint32_t pyr_floats(int32_t width, int32_t height) {
+inline uint32_t pyr_tiles(int32_t width, int32_t height) {
     uint64_t n = 0;
     uint32_t w = ((uint32_t)width + 7u) >> 3, h = ((uint32_t)height + 7u) >> 3;
     for (int l = 0; l < kPyrLevels; ++l) {
@@ -119,7 +119,7 @@ struct IntegrateArgs {
     DepthPyr pyr;            // of the pass's frames
     unsigned int* status;    // streamed pass: the volume's status word (kStatusWaitExpired)
     int32_t hold_first_copy; // streamed pass, failure injection: CTA 0 issues no copy for its first brick
-    int32_t pad1;
+    int32_t layer_runs;      // pass kernels: 4 voxels along z per thread instead of along x
     FrameDesc frames[GBT_MAX_FRAMES_PER_PASS];
 };
 
@@ -154,11 +154,12 @@ struct BatchScene {
 };
 
 struct BatchArgs {
+    VolDesc vol;            // the first scene's volume
     const BatchScene* scenes;
     const FrameDesc* frames;
     int32_t nscenes;        // scenes with frames in this window
     int32_t w0, wn;         // frame window
-    int32_t rows_of_4;      // 1: every scene's x extent is a multiple of 4
+    int32_t layers_of_4;    // 1: every scene's z extent is a multiple of 4
     long long total_bricks; // bricks of those scenes
     DepthPyr pyr;           // of the frame table's frames
     unsigned int* ticket;   // this launch's ticket, zero at launch
@@ -292,7 +293,8 @@ cudaError_t launch_weld_vertices_fixed(const WeldArgs& a, cudaStream_t s);
 cudaError_t launch_batch_compat_ref(const BatchArgs& a, int brick, int grid, cudaStream_t s);
 // CTAs per SM that the (batched or pass) integrate kernel of a brick shape keeps resident.
 // kind: 0 pass kernel culling a frame per lane, 1 pass kernel culling a brick per lane, 2 batched kernel,
-// 3 kind 1 with the depth staged in shared memory, 4 the streamed pass kernel (brick ignored).
+// 3 kind 1 with the depth staged in shared memory, 4 the streamed pass kernel (brick ignored), 5 kind 1 with
+// voxels along z.
 int integrate_resident_ctas_compat_ref(int kind, int brick);
 int integrate_resident_ctas_compat_ieee(int kind, int brick);
 int integrate_resident_ctas_fixed(int kind, int brick);
@@ -308,10 +310,9 @@ cudaError_t launch_stream_compat_ieee(const IntegrateArgs& a, const VolumeMaps& 
 cudaError_t launch_stream_fixed(const IntegrateArgs& a, const VolumeMaps& m, int grid, cudaStream_t s);
 // k_depth.cu: the depth pyramids of frames [0, n) of a table in device memory, or
 // of a pass's (by value).
-cudaError_t launch_depth_pyramids(const FrameDesc* frames, int n, int32_t max_width, int32_t max_height, float cap,
+cudaError_t launch_depth_pyramids(const FrameDesc* frames, int n, int32_t max_width, int32_t max_height,
                                   const DepthPyr& pyr, cudaStream_t s);
-cudaError_t launch_depth_pyramids(const IntegrateArgs& a, int32_t max_width, int32_t max_height, float cap,
-                                  cudaStream_t s);
+cudaError_t launch_depth_pyramids(const IntegrateArgs& a, int32_t max_width, int32_t max_height, cudaStream_t s);
 // k_util.cu: volume initialisation and the packed per-voxel transform records.
 cudaError_t launch_volume_init(float* D, float* W, int64_t n, float trunc, cudaStream_t s);
 cudaError_t launch_tvoxels(void* out, const VolDesc& v, cudaStream_t s);

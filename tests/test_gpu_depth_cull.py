@@ -39,6 +39,9 @@ def frames(path, fmt, seed, n=16):
             d[rng.random(d.shape) < 0.3] = np.nan
             d[rng.random(d.shape) < 0.1] = np.inf
             d[rng.random(d.shape) < 0.1] = -1.0
+        if fmt == "f32" and k == 8:
+            d[rng.random(d.shape) < 0.01] = 1e-40            # subnormal: 0 where the arithmetic flushes
+            d[rng.random(d.shape) < 0.01] = -0.0
         if k == 5:
             d = d[:203, :317]                                # rows that start anywhere
         if k == 6:
@@ -137,3 +140,37 @@ def test_graph_capture_before_and_after_pyramids_have_room(gpu):
         g.replay()
         D, W = volume_bits(gpu, vol)
         assert np.array_equal(D, want[0]) and np.array_equal(W, want[1])
+
+
+@pytest.mark.parametrize("nz", [1, 3, 4, 5, 71])
+@pytest.mark.parametrize("nx", [1, 31, 36, 65])
+@pytest.mark.parametrize("mode,arith", [("compat", "ieee"), ("fixed", "ieee"), ("compat", "reference")])
+def test_voxel_runs_along_x_and_z(gpu, oracle, nx, nz, mode, arith):
+    """Passes whose threads hold voxels along x or along z, and the batched
+    kernel (along z) of one and of two volumes, at extents around their runs."""
+    depths, poses, cam = frames("circle", "u16", 5, n=9)
+    depths = [d for d in depths if d.shape == depths[0].shape]
+    poses = poses[:len(depths)]
+    tc = config("circle", (nx, 18, nz), cam, mode=mode, arith=arith)
+    dd = [dev_depth(gpu, d) for d in depths]
+    want = TSDFVolume(tc)
+    for d, p in zip(dd, poses):
+        want.integrate_frames([d], [p], brick=5)
+    D0, W0 = volume_bits(gpu, want)
+    for k in (1, 2, 5, 6):
+        vol = TSDFVolume(tc)
+        vol.integrate_sequence(dd, poses, frames_per_pass=k, brick=k % 4)
+        D, W = volume_bits(gpu, vol)
+        assert np.array_equal(W, W0) and np.array_equal(D, D0), k
+    vols = [TSDFVolume(tc), TSDFVolume(config("circle", (40, 18, 8), cam, mode=mode, arith=arith))]
+    for n in (1, 2):
+        for vol in vols:
+            vol.reset()
+        for brick in range(4):
+            vols[0].reset()
+            BatchIntegrator(2, 64).integrate(vols[:n], [dd] * n, [poses] * n, brick=brick)
+            D, W = volume_bits(gpu, vols[0])
+            assert np.array_equal(W, W0) and np.array_equal(D, D0), (n, brick)
+    if arith == "ieee":
+        Do, Wo = oracle_run(oracle, tc, depths, poses)
+        assert np.array_equal(W0, Wo) and np.array_equal(D0, Do.view(np.uint32))
