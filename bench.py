@@ -88,6 +88,11 @@ def volume_cfg(args, cam, mode):
                             camera_width=cam.width, camera_height=cam.height, max_weight=128.0, mode=mode)
 
 
+def depth_pyramids(updates, frames, pixels):
+    """Launches of depth pyramids of a call integrating `frames` frames of `pixels` pixels (the engine's rule)."""
+    return int(updates >= 8 << 20 and updates >= frames * (pixels // 2))
+
+
 class ClockSampler:
     """nvidia-smi samples (every 100 ms) of SM clock and throttle reasons
     while running.  Entering waits for nvidia-smi's first sample, so that the
@@ -967,8 +972,9 @@ def multiscene(args, torch, rank, world, local):
         "per_scene": per_scene,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "ms_per_step": 1e3 * float(np.mean(e2e))},
-        # per step: a reset per volume, the batched launches, five mesh launches per volume
-        "gpu_launches": args.steps * (6 * len(vols) + ((max(nfs) + fpl - 1) // fpl)),
+        # per step: a reset per volume, the depth pyramids, the batched launches, five mesh launches per volume
+        "gpu_launches": args.steps * (6 * len(vols) + ((max(nfs) + fpl - 1) // fpl) +
+                                      depth_pyramids(updates, sum(nfs), cam.width * cam.height)),
         "clocks": clocks.summary(),
         "autotune": {"candidates": len(table)},
     }
@@ -1301,14 +1307,15 @@ def main():
     frame_px = cam.width * cam.height
     alg_bytes = 16.0 * nvox + (nf / n_passes) * frame_px * 2 + (nf / n_passes) * 64
     achieved = alg_bytes / (launch_ms * 1e-3) / 1e9
-    # DRAM bytes and warp instructions: one ncu capture of the five
+    # DRAM bytes and warp instructions: one ncu capture of the three
     # integrate_batch_kernel launches of a step of this workload (512^3, 300
-    # frames in windows of 64 and 44, brick 2, resident CTAs): 4.372 GB read +
-    # 3.176 GB written and 28.17 G warp instructions for the step (bricks no
-    # frame sees are neither loaded nor stored).  Only for that launch shape;
-    # other grids, shapes and the fixed mode were not captured.
-    captured = (path == "batched" and args.mode == "compat" and args.grid == 512 and nf == 300 and K == 64)
-    traffic = (4.37171e9 + 3.17576e9) / n_passes if captured else None
+    # frames in windows of 128, resident CTAs), per brick; bricks that no frame
+    # can update are neither loaded nor stored.  Only for those launch shapes;
+    # other grids, windows and the fixed mode were not captured.
+    captures = {1: (4.00668e9 + 2.21200e9, 16.47433e9), 2: (3.69794e9 + 2.17665e9, 17.26246e9)}
+    captured = (path == "batched" and args.mode == "compat" and args.grid == 512 and nf == 300 and K == 128 and
+                brick in captures)
+    traffic = captures[brick][0] / n_passes if captured else None
     peak, peak_kind = peaks()
     # The kernel is bound by instruction issue, not by HBM (a window of K
     # frames shares each voxel's 16 bytes).  Its issue roofline: the captured
@@ -1317,7 +1324,7 @@ def main():
     # SM at the median SM clock sampled while timing.
     issue = None
     if captured:
-        warp_inst_per_update = 28.16625e9 / (512 ** 3 * 300)
+        warp_inst_per_update = captures[brick][1] / (512 ** 3 * 300)
         sm_count = torch.cuda.get_device_properties(local).multi_processor_count
         sm_mhz = (clocks.summary().get("sm_mhz") or 0.0)
         upd_per_s = nvox * (nf / n_passes) / (launch_ms * 1e-3)
@@ -1432,8 +1439,12 @@ def main():
         "mesh": {"triangles_per_s": ntri / (float(np.mean(mesh_ms)) * 1e-3) if ntri else 0.0, "triangles": ntri},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "ms_per_step": float(np.mean(e2e_ms))},
-        # per step: reset, the integrate launches, five mesh launches (bits, count, reduce, scan, emit)
-        "gpu_launches": args.steps * (1 + n_passes + 5),
+        # per step: reset, the integrate launches and their depth pyramids (one per call: the batch, or each
+        # pass), five mesh launches (bits, count, reduce, scan, emit)
+        "gpu_launches": args.steps * (1 + n_passes + 5 + (
+            depth_pyramids(nvox * nf, nf, frame_px) if path == "batched" else
+            0 if brick >= 4 else sum(depth_pyramids(nvox * k, k, frame_px)
+                                     for k in [K] * (nf // K) + [nf % K] * (nf % K > 0)))),
         "clocks": clocks.summary(),
         "wall_s_timed": t_wall,
         "autotune": {"ns_per_update": tune["ns_per_update"], "candidates": candidates},

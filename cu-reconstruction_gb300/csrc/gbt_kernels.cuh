@@ -74,6 +74,8 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
     asm("fma.rn" GBT_F2_FTZ ".f32x2 %0, %1, %2, %3;" : "=l"(d.r) : "l"(a.r), "l"(b.r), "l"(c.r));
     return d;
 }
+// (A paired add whose only input is one paired product is contracted with it, the
+// _rn of both notwithstanding: such sums are written with scalar adds.)
 __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
     f2 d;
     asm("mul.rn" GBT_F2_FTZ ".f32x2 %0, %1, %2;" : "=l"(d.r) : "l"(a.r), "l"(b.r));
@@ -399,9 +401,9 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
 }
 
 // ---------------------------------------------------------------------------
-// Integrate.  One CTA of 128 threads works on a brick of (4*TX) x BY x BZ
-// voxels; a thread owns 4 consecutive voxels along x, moved as one 16-byte
-// load/store of distance and one of weight.  All frames of the pass are
+// Integrate.  One CTA of 128 threads works on a brick of BX x BY x BZ voxels; a
+// thread owns 4 consecutive voxels along x, moved as one 16-byte load/store of
+// distance and one of weight, or along z (BrickLayout).  All frames of the pass are
 // applied to the voxels in registers, in frame order, so a voxel sees exactly
 // the sequence of updates the per-frame reference loop would apply.
 
@@ -791,8 +793,9 @@ __device__ __forceinline__ void fixed_store(float tsdf, float max_weight, float&
     w = fminf(__fadd_rn(w, 1.0f), max_weight);
 }
 // Four of them in pairs, for weights of 0 .. 2^22 (2^23 added towards zero leaves a
-// weight's whole part), without a branch per voxel, the conversions and a table of reciprocals in shared memory: eight scenes of 256^3 with 60 frames
-// each 2.22 -> 2.03 ms, one frame at 512^3 172.6 -> 163.4 us.
+// weight's whole part), without a branch per voxel, the conversions and a table of
+// reciprocals in shared memory: eight scenes of 256^3 with 60 frames each 2.22 ->
+// 2.03 ms, one frame at 512^3 172.6 -> 163.4 us.
 __device__ __forceinline__ void fixed_store4(const f2 (&tsdf)[2], const bool (&ok)[4], float max_weight, float* d,
                                              float* w) {
     // (a NaN among the weights makes the sum NaN)
