@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(256) pyramid_table_kernel(const FrameDesc* fra
 }
 
 __global__ void __launch_bounds__(256) pyramid_pass_kernel(const __grid_constant__ IntegrateArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;");   // the pass kernel's CTAs may take their places
     pyramid_block(a.frames[blockIdx.z], const_cast<float2*>(a.pyr.of((int)blockIdx.z)));
 }
 
