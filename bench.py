@@ -90,7 +90,7 @@ def volume_cfg(args, cam, mode):
 
 def depth_pyramids(updates, frames, pixels):
     """Launches of depth pyramids of a call integrating `frames` frames of `pixels` pixels (the engine's rule)."""
-    return int(updates >= 8 << 20 and updates >= frames * (pixels // 2))
+    return int(updates >= (12 if frames == 1 else 8) << 20 and updates >= frames * (pixels // 2))
 
 
 class ClockSampler:
