@@ -92,7 +92,14 @@ protected:
 private:
     bool project(cv::cuda::PtrStepSzb* color, cv::cuda::PtrStepSzf depth, const std::array<r64, 7>& camera_pose);
 
+    // whether the buffer holds every point that is counted (logs as `method` if not)
+    bool counts_points(const char* method) const;
+
+    // the points of num_pts that the buffer holds
+    inline ui64 held_pts() const { return num_pts < capacity ? num_pts : capacity; }
+
     Vertex* device_pts;
+    ui64 capacity;   // points that device_pts has room for
     ui64 num_pts;
     ui64 total_num_pts;
     std::array<r64, 9> camera_matrix;

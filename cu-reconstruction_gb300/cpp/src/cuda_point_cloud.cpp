@@ -22,7 +22,7 @@ void log_engine(const char* where) { std::fprintf(stderr, "[cuda]   %s -- %s\n",
 }  // namespace
 
 cudaPointCloud::cudaPointCloud(const std::array<r64, 9>& camera_param, const size_t total_number_pts)
-    : device_pts(nullptr), num_pts(0), total_num_pts(0), hasRGB(false) {
+    : device_pts(nullptr), capacity(0), num_pts(0), total_num_pts(0), hasRGB(false) {
     camera_matrix = camera_param;
     if (!reserve_memory(total_number_pts)) {
         std::fprintf(stderr, "[cuda]   cudaPointCloud::reserve_memory() -- can't allocate query CUDA memory %lu\n",
@@ -42,26 +42,38 @@ cudaPointCloud::Ptr cudaPointCloud::merge(const cudaPointCloud::Ptr pc1, const c
     const ui64 query_num_pts = pc1->get_num_points() + pc2->get_num_points();
     cudaPointCloud::Ptr cuda_pc = cudaPointCloud::create(pc1->get_camera_parameters(), query_num_pts);
     Vertex* cuda_pts = cuda_pc->get_points();
-    cudaMemcpy(cuda_pts, pc1->get_points(), pc1->get_size(), cudaMemcpyDefault);
-    cudaMemcpy(cuda_pts + pc1->get_num_points(), pc2->get_points(), pc2->get_size(), cudaMemcpyDefault);
+    cudaMemcpy(cuda_pts, pc1->get_points(), pc1->held_pts() * sizeof(Vertex), cudaMemcpyDefault);
+    cudaMemcpy(cuda_pts + pc1->get_num_points(), pc2->get_points(), pc2->held_pts() * sizeof(Vertex), cudaMemcpyDefault);
     cuda_pc->set_total_number_pts();
     return cuda_pc;
 }
 
 void cudaPointCloud::clear() {
-    if (device_pts != nullptr) cudaMemset(device_pts, 0, get_size());
+    if (device_pts != nullptr) cudaMemset(device_pts, 0, held_pts() * sizeof(Vertex));
     num_pts = 0;
 }
 
 void cudaPointCloud::free() {
     if (device_pts != nullptr) cudaFree(device_pts);
     device_pts = nullptr;
+    capacity = 0;
     num_pts = 0;
+}
+
+// Points may be counted that are not there: extract_points counts a slot that
+// it writes again once more, and set_total_number_pts the size that the cloud
+// had before filter_depth or free.  Kernels and loops over them would run past
+// the buffer.
+bool cudaPointCloud::counts_points(const char* method) const {
+    if (num_pts <= capacity) return true;
+    std::fprintf(stderr, "[cuda]   cudaPointCloud::%s() -- %lu points counted, %lu held\n", method,
+                 (unsigned long)num_pts, (unsigned long)capacity);
+    return false;
 }
 
 bool cudaPointCloud::reserve_memory(const ui64 query_number_points) {
     if (query_number_points <= 0) return true;
-    if (query_number_points <= num_pts && device_pts != nullptr) {
+    if (query_number_points <= held_pts() && device_pts != nullptr) {
         clear();
         return true;
     }
@@ -70,6 +82,7 @@ bool cudaPointCloud::reserve_memory(const ui64 query_number_points) {
         device_pts = nullptr;
         return false;
     }
+    capacity = query_number_points;
     // a fresh cloud reads as zero points, as the reference's zeroed managed pages do
     cudaMemset(device_pts, 0, query_number_points * sizeof(Vertex));
     cudaDeviceSynchronize();
@@ -93,7 +106,8 @@ bool cudaPointCloud::extract_points(const cv::cuda::PtrStepSzf depth, const cv::
     const gbt_status st =
         gbt_points_extract(camera_matrix.data(), depth.data, (int64_t)depth.step, GBT_DEPTH_F32_M, 1.0f,
                            colors.data, (int64_t)colors.step, (int32_t)width, (int32_t)height, T.data(), start_idx,
-                           reinterpret_cast<gbt_point*>(device_pts), (int64_t)total_num_pts, nullptr);
+                           reinterpret_cast<gbt_point*>(device_pts),
+                           (int64_t)(total_num_pts < capacity ? total_num_pts : capacity), nullptr);
     if (st != GBT_OK) {
         log_engine("cudaPointCloud::extract_points() -- failed to extract point cloud with CUDA");
         return false;
@@ -105,6 +119,7 @@ bool cudaPointCloud::extract_points(const cv::cuda::PtrStepSzf depth, const cv::
 
 bool cudaPointCloud::project(cv::cuda::PtrStepSzb* color, cv::cuda::PtrStepSzf depth,
                              const std::array<r64, 7>& camera_pose) {
+    if (!counts_points("project_to_depth")) return false;
     const size_t bytes = GBT_POINTS_PROJECT_SCRATCH_BYTES(depth.cols, depth.rows);
     void* scratch = nullptr;
     if (cudaMalloc(&scratch, bytes) != cudaSuccess) {
@@ -159,6 +174,7 @@ bool cudaPointCloud::transform(const std::array<r64, 7>& T) {
         log_error("cudaPointCloud::transform() -- the device points is not allocated");
         return false;
     }
+    if (!counts_points("transform")) return false;
     if (gbt_points_transform(reinterpret_cast<gbt_point*>(device_pts), (int64_t)num_pts, T.data(), nullptr) !=
         GBT_OK) {
         log_engine("cudaPointCloud::transform() -- failed to transform point cloud with CUDA");
@@ -169,7 +185,7 @@ bool cudaPointCloud::transform(const std::array<r64, 7>& T) {
 }
 
 bool cudaPointCloud::add_vertex(const Vertex& v, const ui64 idx) {
-    if (idx >= total_num_pts) {
+    if (idx >= total_num_pts || idx >= capacity) {
         log_error("cudaPointCloud::add_vertex() -- index out of range");
         return false;
     }
@@ -178,7 +194,7 @@ bool cudaPointCloud::add_vertex(const Vertex& v, const ui64 idx) {
 }
 
 bool cudaPointCloud::add_vertex(const float3 pos, const uchar3 color, const ui64 idx, const float4 normal) {
-    if (idx >= total_num_pts) {
+    if (idx >= total_num_pts || idx >= capacity) {
         log_error("cudaPointCloud::add_vertex() -- index out of range");
         return false;
     }
@@ -193,8 +209,9 @@ bool cudaPointCloud::add_vertex(const float3 pos, const uchar3 color, const ui64
 void cudaPointCloud::filter_depth(const r32 depth_threshold_min, const r32 depth_threshold_max) {
     cudaDeviceSynchronize();
     std::vector<Vertex> kept;
-    kept.reserve(num_pts);
-    for (ui64 i = 0; i < num_pts; ++i) {
+    const ui64 n = held_pts();
+    kept.reserve(n);
+    for (ui64 i = 0; i < n; ++i) {
         const r32 z = device_pts[i].pos.z;
         const bool inside = z > depth_threshold_min && z < depth_threshold_max;
         if (!inside) kept.push_back(device_pts[i]);
@@ -208,10 +225,12 @@ void cudaPointCloud::filter_depth(const r32 depth_threshold_min, const r32 depth
     if (!kept.empty()) std::memcpy(out, kept.data(), kept.size() * sizeof(Vertex));
     free();
     device_pts = out;
+    capacity = kept.size();
     num_pts = kept.size();
 }
 
 bool cudaPointCloud::add_point_cloud(const cudaPointCloud::Ptr cuda_pc) {
+    if (!counts_points("add_point_cloud") || !cuda_pc->counts_points("add_point_cloud")) return false;
     const ui64 query_num_pts = cuda_pc->get_num_points() + num_pts;
     Vertex* cuda_pts = nullptr;
     if (cudaMallocManaged(&cuda_pts, query_num_pts * sizeof(Vertex), cudaMemAttachGlobal) != cudaSuccess) return false;
@@ -219,6 +238,7 @@ bool cudaPointCloud::add_point_cloud(const cudaPointCloud::Ptr cuda_pc) {
     cudaMemcpy(cuda_pts + num_pts, cuda_pc->get_points(), cuda_pc->get_size(), cudaMemcpyDefault);
     free();
     device_pts = cuda_pts;
+    capacity = query_num_pts;
     num_pts = query_num_pts;
     total_num_pts = query_num_pts;
     return true;
@@ -237,6 +257,7 @@ bool cudaPointCloud::save_ply(const std::string& filepath) const {
         return false;
     }
     cudaDeviceSynchronize();
+    const ui64 n = held_pts();
     std::ofstream out(filepath.c_str());
     static const char* const kHeader[] = {"ply", "format ascii 1.0", nullptr, "property float x", "property float y",
                                           "property float z", "property uchar red", "property uchar green",
@@ -245,9 +266,9 @@ bool cudaPointCloud::save_ply(const std::string& filepath) const {
         if (line)
             out << line << '\n';
         else
-            out << "element vertex " << num_pts << '\n';
+            out << "element vertex " << n << '\n';
     }
-    for (ui64 i = 0; i < num_pts; ++i) {
+    for (ui64 i = 0; i < n; ++i) {
         const Vertex& v = device_pts[i];
         out << v.pos.x << ' ' << v.pos.y * -1.f << ' ' << v.pos.z * -1.f << ' ' << (i32)v.color.x << ' '
             << (i32)v.color.y << ' ' << (i32)v.color.z << '\n';

@@ -94,6 +94,16 @@ class PointCloud:
         """The points as a structured array (fields pos, normal, color, class_id)."""
         return self.get_points().cpu().numpy().reshape(-1).view(POINT_DTYPE)
 
+    def _counts_points(self, method):
+        """Whether the cloud holds every point that it counts.  It need not:
+        extract_points counts a slot it writes again once more, and
+        set_total_number_pts the size that a cloud had before filter_depth.  The
+        kernels would read and write past the points."""
+        if self.num_pts <= self.device_pts.shape[0]:
+            return True
+        _log("cudaPointCloud::%s() -- %d points counted, %d held" % (method, self.num_pts, self.device_pts.shape[0]))
+        return False
+
     # -- kernels ----------------------------------------------------------------
     def extract_points(self, depth, colors, transform, frame_idx, depth_scale=0.001, stream=None):
         """cudaPointCloud::extract_points (cuda_point_cloud.cu:179-226): depth (H, W)
@@ -121,7 +131,8 @@ class PointCloud:
         st = L.lib().gbt_points_extract(C.byref(_k9(self.camera_matrix)), depth.data_ptr(),
                                         depth.stride(0) * (4 if f32 else 2), L.DEPTH_F32_M if f32 else L.DEPTH_U16,
                                         float(depth_scale), cptr, cpitch, W, H, C.byref(_pose7(transform)), start,
-                                        self.device_pts.data_ptr(), self.total_num_pts, _stream_handle(stream))
+                                        self.device_pts.data_ptr(), min(self.total_num_pts, self.device_pts.shape[0]),
+                                        _stream_handle(stream))
         if st != L.GBT_OK:
             _log("cudaPointCloud::extract_points() -- " + L.lib().gbt_last_error().decode())
             return False
@@ -129,6 +140,8 @@ class PointCloud:
         return True
 
     def _project(self, color, depth, camera_pose, stream):
+        if not self._counts_points("project_to_depth"):
+            return False
         torch = _torch()
         L.device_image(depth, "depth", (torch.float32,))
         H, W = int(depth.shape[0]), int(depth.shape[1])
@@ -174,6 +187,8 @@ class PointCloud:
         """cudaPointCloud::transform (cuda_point_cloud.cu:356-385)."""
         if self.num_pts == 0:
             _log("cudaPointCloud::transform() -- the number of points is 0")
+            return False
+        if not self._counts_points("transform"):
             return False
         st = L.lib().gbt_points_transform(C.c_void_p(self.device_pts.data_ptr()), self.num_pts,
                                           C.byref(_pose7(T)), _stream_handle(stream))
@@ -235,7 +250,7 @@ class PointCloud:
         with open(filepath, "w") as f:
             f.write("ply\nformat ascii 1.0\nelement vertex %d\nproperty float x\nproperty float y\n"
                     "property float z\nproperty uchar red\nproperty uchar green\nproperty uchar blue\n"
-                    "end_header\n" % self.num_pts)
+                    "end_header\n" % len(v))
             for p, c in zip(v["pos"], v["color"]):
                 f.write("%g %g %g %d %d %d\n" % (p[0], p[1] * np.float32(-1), p[2] * np.float32(-1), c[0], c[1], c[2]))
         return True
