@@ -32,6 +32,8 @@ struct VolDesc {
     float max_depth;
     float min_z;
     float fx, fy, cx, cy;
+    float clear;   // least distance from the camera plane at which boxes are tested (add_clear in capi.cu)
+    int32_t pad1;
 };
 
 // One frame as the kernels see it.  q/t: the reference's float quaternion
@@ -54,10 +56,10 @@ enum SlotFormat : int32_t {
     kSlotU16Mul = 2,  // uint16 x scale as a conversion and a multiply (any other scale)
 };
 
-// A frame as the integrate kernels keep it in shared memory (96 bytes, six
+// A frame as the integrate kernels keep it in shared memory (80 bytes, five
 // 16-byte words): pose table entry, depth image, its row pitch in elements,
-// the sample format, the depth scale in both halves of a paired-FP32 operand,
-// and the box test's margins (set_limits).
+// the sample format and the depth scale in both halves of a paired-FP32
+// operand.
 struct __align__(16) FrameSlot {
     float pose[12];
     const void* depth;
@@ -65,9 +67,8 @@ struct __align__(16) FrameSlot {
     int32_t fmt;
     unsigned long long scale2;
     uint32_t width, height;
-    float eps, clear, pad0, pad1;
 };
-static_assert(sizeof(FrameSlot) == 96, "six 16-byte words");
+static_assert(sizeof(FrameSlot) == 80, "five 16-byte words");
 
 // Unsigned 32-bit division by a run-time invariant divisor with one
 // multiply-high, after Granlund & Montgomery, "Division by invariant integers

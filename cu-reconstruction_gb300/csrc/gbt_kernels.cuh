@@ -177,7 +177,7 @@ __device__ __forceinline__ bool div2_safe(f2 n0, f2 n1, f2 w0, f2 w1) {
     return fminf(fminf(a, b), fminf(c, d)) >= 0x1p-80f && fmaxf(fmaxf(a, b), fmaxf(c, d)) <= 0x1p80f && lo >= 0.5f &&
            hi <= 0x1p24f;
 }
-// INSIDE: 1e-4 < |z| < 1e7, and u and v are in an image of at least 4 x 4 pixels
+// INSIDE: 1e-4 < |z| < 1e9, and u and v are in an image of at least 4 x 4 pixels
 // with 2 to spare (a quotient too small for div2 then changes no sum).
 template <bool INSIDE>
 __device__ __forceinline__ void compat_proj2(f2 cx, f2 cy, f2 cz, float fx, float fy, float ccx, float ccy, f2& qu,
@@ -243,9 +243,9 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 // What a frame can do to a box of voxels, evaluated by one thread.  The test is
 // conservative: it only reports kBoxCulled when every voxel of the box is certain to be rejected by
 // the per-voxel test (the projected box lies in the convex hull of its
-// projected corners when no corner is near the camera plane, as far away as the
-// rounding of its coordinates asks), with a margin of two pixels and 1e-4 in depth
-// that covers rounding.
+// projected corners when no corner is near the camera plane: nearer than v.clear,
+// which depends on the rounding of the frames' coordinates, add_clear in capi.cu),
+// with a margin of two pixels and 1e-4 in depth that covers rounding.
 //
 // With the frame's depth pyramid (`pyr`, NULL: none; k_depth.cu) it also culls
 // boxes that the frame's depth cannot update: those whose pixels, taken as the
@@ -268,39 +268,17 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 // KINDS false: only kBoxCulled is told from kBoxAny.
 enum { kBoxCulled = 0, kBoxAny = 1, kBoxInside = 2, kBoxFront = 3 };
 
-// How near the camera plane a frame's projections of a volume are accurate, and the
-// margin of its depths.  With `reach` the largest term of a camera coordinate and
-// `span` that of u z and v z, those are off by less than 1e-6 of them (a dozen
-// roundings of 2^-24), at the corners of a box and in a voxel's own evaluation.  So
-// from z = clear on, 250 times its error, u and v are within half a pixel in both
-// (two centimetres for a room of five metres).  Once per frame: formed anew in every
-// test, one-frame passes took 1 to 2 % longer.
-template <int MODE>
-__device__ __forceinline__ void set_limits(const VolDesc& v, FrameSlot& fs) {
-    const float* fr = fs.pose;
-    const int n[3] = {v.nx, v.ny, v.nz};
-    float xyz = 0.f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        xyz = fmaxf(xyz, fmaxf(fabsf(centre(0, v.vs[k], v.off[k])), fabsf(centre(n[k] - 1, v.vs[k], v.off[k]))));
-    const float focal = fmaxf(fabsf(v.fx), fabsf(v.fy)) + fmaxf(fabsf(v.cx), fabsf(v.cy));
-    const float size = fmaxf((float)fs.width, (float)fs.height);
-    float reach, span;
-    if (MODE == kCompat) {
-        float r = 1.f;   // (quaternions are not normalised)
-#pragma unroll
-        for (int k = 0; k < 9; ++k) r = fmaxf(r, fabsf(fr[k]));
-        reach = fmaxf(r * xyz, fmaxf(fabsf(fr[9]), fmaxf(fabsf(fr[10]), fabsf(fr[11]))));
-        span = reach * (focal + size);
-    } else {
-        reach = fmaxf(xyz, fabsf(fr[11]));
-        span = fmaxf(focal * xyz, fmaxf(fabsf(fr[3]), fabsf(fr[7]))) + reach * size;
-    }
-    fs.eps = 1e-4f + 1e-5f * reach;
-    fs.clear = fmaxf(fs.eps, fmaxf(4e-3f * reach, 2e-6f * span));
-}
-
-template <int MODE, bool KINDS>
+// OWN: kBoxInside asks for the limits of the box's own coordinates.  Otherwise those
+// of v.clear, which is no less sound (u and v within a pixel, with two to spare, and
+// z well above 1e-4).  The difference is in the registers that the compiler gives
+// the kernels around it: reference arithmetic's batched kernel keeps 56 without (300
+// frames at 512^3 19.0 against 19.4 ms), the passes 64 to 72 with.
+#if defined(GBT_REF_ARITH)
+constexpr bool kBatchOwn = false;
+#else
+constexpr bool kBatchOwn = true;
+#endif
+template <int MODE, bool KINDS, bool OWN = true>
 __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, const float2* pyr, int x_lo, int x_hi,
                                         int y_lo, int y_hi, int z_lo, int z_hi) {
     const float* fr = fs.pose;
@@ -311,8 +289,22 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
     // the least and the largest z that a voxel's depth is compared with
     float near = MODE == kCompat ? Zw[0] : 3.0e38f, back = MODE == kCompat ? Zw[1] : -3.0e38f;
     int npos = 0, nneg = 0, nbehind = 0;
-    // (boxes that come nearer to the camera plane than `clear` are left to their voxels)
-    const float eps = fs.eps, clear = fs.clear;
+    float zmin = 3.0e38f, zmax = -3.0e38f;
+    // depth margin: far above the float rounding of a camera coordinate at this scale
+    const float tmax = (MODE == kCompat) ? fmaxf(fabsf(fr[9]), fmaxf(fabsf(fr[10]), fabsf(fr[11])))
+                                         : fabsf(fr[11]);
+    const float scale = fmaxf(fmaxf(fmaxf(fabsf(X[0]), fabsf(X[1])), fmaxf(fabsf(Y[0]), fabsf(Y[1]))),
+                              fmaxf(fmaxf(fabsf(Zw[0]), fabsf(Zw[1])), tmax));
+    const float eps = 1e-4f + 1e-5f * scale;
+    // Boxes that come nearer to the camera plane than `clear` are left to their voxels.
+    // (v.clear is no less than eps: the maximum keeps the passes of reference arithmetic
+    // at 64 registers, 217 against 228 us for 32 frames at 192^3; those of IEEE
+    // arithmetic are 1 % faster without it.)
+#if defined(GBT_REF_ARITH)
+    const float clear = fmaxf(eps, v.clear);
+#else
+    const float clear = v.clear;
+#endif
     if (MODE == kCompat) {
         // world z exactly 0 sends a voxel to pixel (0,0) (camera_util.cu:46): keep such boxes
         if (!(Zw[0] > 0.f || Zw[1] < 0.f)) return kBoxAny;
@@ -341,6 +333,10 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
         else if (cz < -clear)
             ++nneg;
         const float rz = 1.0f / cz;
+        if (KINDS) {
+            zmin = fminf(zmin, cz);
+            zmax = fmaxf(zmax, cz);
+        }
         const float u = cx * rz, w = cy * rz;
         umin = fminf(umin, u);
         umax = fmaxf(umax, u);
@@ -367,9 +363,34 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
         inside = true;
     }
     // (coordinates so large that corners may have overflowed are left to the voxels)
-    if (!(eps < 10.f)) return kBoxAny;
+    if (!(scale < 1e6f)) return kBoxAny;
     const float ur = W - 1.f, vr = H - 1.f;
     inside = inside && umin >= 2.f && umax <= ur - 2.f && vmin >= 2.f && vmax <= vr - 2.f;
+    float reach = 0.f;
+    if (KINDS && OWN && inside) {
+        // With `reach` the largest term of a camera coordinate and `span` that of
+        // u z and v z, these are off by less than 1e-6 of them (a dozen roundings
+        // of 2^-24), here and in the voxel's own evaluation: z has to be 250 times
+        // its error, and u and v within half a pixel.
+        const float xyz = fmaxf(fmaxf(fmaxf(fabsf(X[0]), fabsf(X[1])), fmaxf(fabsf(Y[0]), fabsf(Y[1]))),
+                                fmaxf(fabsf(Zw[0]), fabsf(Zw[1])));
+        float span;
+        if (MODE == kCompat) {
+            float r = 1.f;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) r = fmaxf(r, fabsf(fr[k]));
+            reach = fmaxf(r * xyz, tmax);
+            span = reach * (fmaxf(fabsf(v.fx), fabsf(v.fy)) + fmaxf(fabsf(v.cx), fabsf(v.cy)) + fmaxf(W, H));
+        } else {
+            const float r = fmaxf(fmaxf(1.f, fabsf(fr[8])), fmaxf(fabsf(fr[9]), fabsf(fr[10])));
+            const float p = fmaxf(fmaxf(fmaxf(fabsf(fr[0]), fabsf(fr[1])), fmaxf(fabsf(fr[2]), fabsf(fr[4]))),
+                                  fmaxf(fabsf(fr[5]), fabsf(fr[6])));
+            reach = fmaxf(r * xyz, tmax);
+            span = fmaxf(p * xyz, fmaxf(fabsf(fr[3]), fabsf(fr[7]))) + reach * fmaxf(W, H);
+        }
+        const float z = zmin > 0.f ? zmin : -zmax;   // (the corners are on one side of the camera)
+        inside = z >= 4e-3f * reach && z >= 2e-6f * span && fmaxf(fabsf(zmin), fabsf(zmax)) < 1e9f;
+    }
     const int open = KINDS && inside ? kBoxInside : kBoxAny;
     if (!pyr) return open;
     const uint32_t a = (uint32_t)fminf(fmaxf(umin - 2.f, 0.f), ur), b = (uint32_t)fminf(fmaxf(umax + 2.f, 0.f), ur);
@@ -397,7 +418,7 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
         }
     if (!(far > 0.f) || far + v.trunc + 2.f * eps < near) return kBoxCulled;
     const float cap = MODE == kFixed ? v.max_depth : 24.0f;
-    if (KINDS && inside && far <= cap && fs.fmt != kSlotU16Mul && least - back >= v.trunc + 4.f * eps)
+    if (KINDS && inside && far <= cap && fs.fmt != kSlotU16Mul && least - back >= v.trunc + (OWN ? 2.f * eps + 2e-5f * reach : 4.f * eps))
         return kBoxFront;
     return open;
 }
@@ -414,7 +435,7 @@ __device__ __forceinline__ int box_test(const VolDesc& v, const FrameSlot& fs, c
 // K[R|t]) and the image description in the form the per-voxel code uses, so
 // that a thread reads a frame's constants with a few broadcast shared loads.
 template <int MODE>
-__device__ __forceinline__ void load_slot(const VolDesc& v, const FrameDesc& fd, FrameSlot& s) {
+__device__ __forceinline__ void load_slot(const FrameDesc& fd, FrameSlot& s) {
     if (MODE == kCompat) {
         float R[9];
         compat_rotation(fd.q, R);
@@ -437,7 +458,6 @@ __device__ __forceinline__ void load_slot(const VolDesc& v, const FrameDesc& fd,
     s.scale2 = f2_splat(fd.scale).r;
     s.width = (uint32_t)fd.width;
     s.height = (uint32_t)fd.height;
-    set_limits<MODE>(v, s);
 }
 
 // The bits of the thread's 4 depth samples, 0 where `in` is false: a uint16
@@ -1135,7 +1155,7 @@ __global__ void __launch_bounds__(128, LANE_BRICKS && !Z ? 10 : 0) integrate_ker
     const VolDesc& v = a.vol;
     const int tid = threadIdx.x;
     const int nf = a.nframes;
-    if (tid < nf) load_slot<MODE>(v, a.frames[tid], s_frame[tid]);
+    if (tid < nf) load_slot<MODE>(a.frames[tid], s_frame[tid]);
     __syncthreads();
     grid_wait();   // (everything before reads the launch arguments only)
 
@@ -1345,7 +1365,7 @@ __global__ void __launch_bounds__(128) integrate_stream_kernel(const __grid_cons
     const VolDesc& v = a.vol;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nf = a.nframes;
-    if (tid < nf) load_slot<MODE>(v, a.frames[tid], s_frame[tid]);
+    if (tid < nf) load_slot<MODE>(a.frames[tid], s_frame[tid]);
     if (tid == 0) {
         for (int st = 0; st < S; ++st) mbar_init(&s_full[st], 1);
         mbar_init_fence();
@@ -1497,7 +1517,7 @@ __global__ void __launch_bounds__(128) integrate_batch_kernel(const __grid_const
         const int nf = min(S.nframes - a.w0, a.wn);
         if (s_scene != scene) {
             scene = s_scene;
-            for (int f = tid; f < nf; f += blockDim.x) load_slot<MODE>(S.vol, frames[f], s_frame[f]);
+            for (int f = tid; f < nf; f += blockDim.x) load_slot<MODE>(frames[f], s_frame[f]);
             if (!ONE && tid == 0) s_vol = S.vol;
             __syncthreads();
         }
@@ -1512,7 +1532,7 @@ __global__ void __launch_bounds__(128) integrate_batch_kernel(const __grid_const
         // tests by each warp were 5 % of the kernel's instructions).
         static_assert(kBatchMaxFrames <= 128, "a thread per frame");
         {
-            const int code = tid < nf ? box_test<MODE, true>(v, s_frame[tid], a.pyr.of(S.first_frame + a.w0 + tid), bx0,
+            const int code = tid < nf ? box_test<MODE, true, kBatchOwn>(v, s_frame[tid], a.pyr.of(S.first_frame + a.w0 + tid), bx0,
                                                        min(bx0 + BX, v.nx) - 1, by0, min(by0 + BY, v.ny) - 1, bz0,
                                                        min(bz0 + BZ, v.nz) - 1)
                                       : kBoxCulled;
