@@ -137,6 +137,7 @@ bool TSDFVolume::integrate(const cv::cuda::PtrStepSzb color, const cv::cuda::Ptr
     f.format = GBT_DEPTH_F32_M;
     f.depth_scale = 1.f;
     for (int k = 0; k < 7; ++k) f.pose[k] = camera_pose[k];
+    gbt_volume_reserve(vol, &f, 1);   // (without the room: the same result in more time)
     if (gbt_integrate(vol, &f, 1, nullptr) != GBT_OK) {
         log_engine_error("TSDFVolume::integrate() -- failed integrate signed distance function on voxels data");
         return false;
@@ -153,6 +154,7 @@ bool TSDFVolume::integrate_frames(const gbt_frame* frames, i32 nframes, cudaStre
     if (!vol) return false;
     for (i32 s = 0; s < nframes; s += GBT_MAX_FRAMES_PER_PASS) {
         const i32 n = nframes - s < GBT_MAX_FRAMES_PER_PASS ? nframes - s : GBT_MAX_FRAMES_PER_PASS;
+        gbt_volume_reserve(vol, frames + s, n);
         if (gbt_integrate(vol, frames + s, n, stream) != GBT_OK) {
             log_engine_error("TSDFVolume::integrate_frames()");
             return false;

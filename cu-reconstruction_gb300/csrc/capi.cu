@@ -85,37 +85,63 @@ int device_sms() {
 
 namespace {
 
+// Launches of depth pyramids and frames that got one (gbt_debug_count).
+std::atomic<int64_t> g_pyramid_launches{0}, g_pyramid_frames{0};
+
 // A volume's or batch's buffer for depth pyramids: at first the end of its own
-// device allocation, a larger one of its own when a call needs it.  Buffers that
-// were outgrown stay until the owner goes, since a captured graph may read them
-// (they add up to less than the last one, which is at least twice as large as
-// the one before).
+// device allocation, a larger one of its own once the caller asks for it
+// (pyr_reserve; the integrate calls take what is there).  Buffers that were
+// outgrown stay until the owner goes, since a captured graph may read them (they
+// add up to less than the last one, which is at least twice as large as the one
+// before, or to kPyrMaxBytes before a last one of that size).
 struct PyrBuffer {
     float2* data;
     size_t tiles;
     void* own[32];   // allocations, the last of them data's
     int nown;
 };
+constexpr size_t kPyrMaxBytes = (size_t)1 << 30;   // 20,000 frames of 640x480
 
-// Room for n tiles, or NULL: the caller then goes without pyramids (an
-// allocation failed, or would be needed while `s` is being captured).
-float2* pyr_room(PyrBuffer* b, size_t n, cudaStream_t s) {
-    if (b->tiles >= n) return b->data;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone || b->nown >= 32) {
+// The pyramids of a call: of frames of up to width x height, `frames` of them.
+struct PyrPlan {
+    int32_t width, height;
+    uint32_t stride;   // tiles per frame; 0: pyramids do not pay
+    uint32_t frames;
+};
+
+// The plan's pyramids in `b`, none if there is no room for all of them.
+gbt::DepthPyr pyr_place(const PyrBuffer& b, const PyrPlan& p) {
+    gbt::DepthPyr d{nullptr, p.stride, 0u};
+    if (p.stride && (size_t)p.stride * p.frames <= b.tiles) d.base = b.data;
+    return d;
+}
+
+void count_pyramids(int64_t frames) {
+    g_pyramid_launches.fetch_add((frames + 65534) / 65535, std::memory_order_relaxed);
+    g_pyramid_frames.fetch_add(frames, std::memory_order_relaxed);
+}
+
+// Room for the plan's pyramids, if they are not too large.
+gbt_status pyr_reserve(PyrBuffer* b, const PyrPlan& p) {
+    constexpr size_t kMax = kPyrMaxBytes / sizeof(float2);
+    const size_t need = (size_t)p.stride * p.frames;
+    if (b->tiles >= need || need > kMax) return GBT_OK;
+    const size_t want = std::min(std::max(need, 2 * b->tiles), kMax);
+    void* p0 = nullptr;
+    // (an allocation is harmless to work that this or another thread captures)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = b->nown < 32 ? dev_alloc(&p0, want * sizeof(float2)) : cudaErrorMemoryAllocation;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
         cudaGetLastError();
-        return nullptr;
+        return fail(GBT_ERR_ALLOC, "allocating %zu bytes for depth pyramids: %s", want * sizeof(float2),
+                    cudaGetErrorString(e));
     }
-    const size_t want = std::max(n, 2 * b->tiles);
-    void* p = nullptr;
-    if (cudaMalloc(&p, want * sizeof(float2)) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    b->own[b->nown++] = p;
-    b->data = static_cast<float2*>(p);
+    b->own[b->nown++] = p0;
+    b->data = static_cast<float2*>(p0);
     b->tiles = want;
-    return b->data;
+    return GBT_OK;
 }
 
 void pyr_free(PyrBuffer* b) {
@@ -277,6 +303,17 @@ void add_clear(const gbt_volume_cfg& c, const gbt::FrameDesc& f, gbt::VolDesc* d
     d->clear = span < 1e30f ? std::max(d->clear, clear) : HUGE_VALF;   // (NaN: every box is left to its voxels)
 }
 
+// The depth pyramids of a pass of checked frames.
+PyrPlan pass_pyramids(const gbt_volume* v, const gbt_frame* frames, int32_t n) {
+    PyrPlan p{0, 0, 0u, (uint32_t)n};
+    for (int i = 0; i < n; ++i) {
+        p.width = std::max(p.width, frames[i].width);
+        p.height = std::max(p.height, frames[i].height);
+    }
+    if (pyramids_pay(v->nvox * n, n, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
+    return p;
+}
+
 // Voxels of a grid, or -1 when there are 2^32 or more (no intermediate
 // product overflows: n0 * n1 < 2^64).
 int64_t grid_voxels(const uint32_t n[3]) {
@@ -384,6 +421,15 @@ gbt_status gbt_debug_inject(int32_t what, int64_t skip, int64_t count) {
             return GBT_OK;
         default:
             return fail(GBT_ERR_INVALID_ARG, "gbt_debug_inject: unknown kind %d", what);
+    }
+}
+
+gbt_status gbt_debug_count(int32_t what, int64_t* value) {
+    if (!value) return fail(GBT_ERR_INVALID_ARG, "gbt_debug_count: value is NULL");
+    switch (what) {
+        case GBT_COUNT_PYRAMID_LAUNCHES: *value = g_pyramid_launches.load(); return GBT_OK;
+        case GBT_COUNT_PYRAMID_FRAMES: *value = g_pyramid_frames.load(); return GBT_OK;
+        default: return fail(GBT_ERR_INVALID_ARG, "gbt_debug_count: unknown count %d", what);
     }
 }
 
@@ -741,18 +787,12 @@ gbt_status gbt_integrate_tuned(gbt_volume* v, const gbt_frame* frames, int32_t n
     cudaError_t e;
     cudaGetLastError();  // a launch reports only its own failure
     if (brick < 4) {
-        int32_t mw = 0, mh = 0;
-        for (int i = 0; i < nframes; ++i) {
-            mw = std::max(mw, frames[i].width);
-            mh = std::max(mh, frames[i].height);
-        }
-        const uint32_t stride = gbt::pyr_tiles(mw, mh);
-        if (stride && pyramids_pay(v->nvox * nframes, nframes, (int64_t)mw * mh))
-            a.pyr.base = pyr_room(&v->pyr, (size_t)stride * (size_t)nframes, as_stream(stream));
+        const PyrPlan p = pass_pyramids(v, frames, nframes);
+        a.pyr = pyr_place(v->pyr, p);
         if (a.pyr.base) {
-            a.pyr.stride = stride;
-            e = gbt::launch_depth_pyramids(a, mw, mh, as_stream(stream));
+            e = gbt::launch_depth_pyramids(a, p.width, p.height, as_stream(stream));
             if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
+            count_pyramids(nframes);
         }
     }
     if (brick == 8) {
@@ -775,6 +815,13 @@ gbt_status gbt_integrate_tuned(gbt_volume* v, const gbt_frame* frames, int32_t n
 
 gbt_status gbt_integrate(gbt_volume* v, const gbt_frame* frames, int32_t nframes, void* stream) {
     return gbt_integrate_tuned(v, frames, nframes, 0, 0, stream);
+}
+
+gbt_status gbt_volume_reserve(gbt_volume* v, const gbt_frame* frames, int32_t nframes) {
+    if (!v) return fail(GBT_ERR_INVALID_ARG, "volume is NULL");
+    const gbt_status st = check_frames(frames, nframes);
+    if (st != GBT_OK) return st;
+    return pyr_reserve(&v->pyr, pass_pyramids(v, frames, nframes));
 }
 
 }  // extern "C"
@@ -953,6 +1000,36 @@ size_t batch_bytes(int32_t max_scenes, int32_t max_frames) {
     return 256 + (size_t)max_scenes * sizeof(gbt::BatchScene) + (size_t)max_frames * sizeof(gbt::FrameDesc);
 }
 
+// The items of a batched call, each by itself.
+gbt_status check_items(const gbt_batch* b, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
+                       int32_t nframes) {
+    if (!b || !items || !frames) return fail(GBT_ERR_INVALID_ARG, "batch, items or frames is NULL");
+    if (nitems < 1 || nitems > b->max_scenes) return fail(GBT_ERR_INVALID_ARG, "nitems %d outside 1..%d", nitems, b->max_scenes);
+    if (nframes < 1 || nframes > b->max_frames)
+        return fail(GBT_ERR_INVALID_ARG, "nframes %d outside 1..%d", nframes, b->max_frames);
+    for (int i = 0; i < nitems; ++i) {
+        const gbt_batch_item& it = items[i];
+        if (!it.volume) return fail(GBT_ERR_INVALID_ARG, "item %d has no volume", i);
+        if (it.nframes < 0 || it.first_frame < 0 || it.first_frame + it.nframes > nframes)
+            return fail(GBT_ERR_INVALID_ARG, "item %d: frames [%d, %d) outside the frame table", i, it.first_frame,
+                        it.first_frame + it.nframes);
+    }
+    return GBT_OK;
+}
+
+// The depth pyramids of a batched call whose items have been checked.
+PyrPlan batch_pyramids(const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames, int32_t nframes) {
+    PyrPlan p{0, 0, 0u, (uint32_t)nframes};
+    for (int i = 0; i < nframes; ++i) {
+        p.width = std::max(p.width, frames[i].width);
+        p.height = std::max(p.height, frames[i].height);
+    }
+    int64_t work = 0;
+    for (int i = 0; i < nitems; ++i) work += items[i].volume->nvox * items[i].nframes;   // (below 2^32 * 2^24)
+    if (pyramids_pay(work, nframes, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
+    return p;
+}
+
 }  // namespace
 
 extern "C" {
@@ -996,30 +1073,33 @@ gbt_status gbt_batch_destroy(gbt_batch* b) {
     return GBT_OK;
 }
 
+gbt_status gbt_batch_reserve(gbt_batch* b, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
+                             int32_t nframes) {
+    const gbt_status st = check_items(b, items, nitems, frames, nframes);
+    if (st != GBT_OK) return st;
+    for (int i = 0; i < nframes; ++i)
+        if (frames[i].width <= 0 || frames[i].height <= 0)
+            return fail(GBT_ERR_INVALID_ARG, "frame %d: depth width/height are zero", i);
+    return pyr_reserve(&b->pyr, batch_pyramids(items, nitems, frames, nframes));
+}
+
 gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
                                int32_t nframes, int32_t frames_per_launch, int32_t brick, int32_t ctas_per_sm,
                                void* stream) {
     gbt::TraceRange trace_("gbt_integrate_batch");
-    if (!b || !items || !frames) return fail(GBT_ERR_INVALID_ARG, "batch, items or frames is NULL");
-    if (nitems < 1 || nitems > b->max_scenes) return fail(GBT_ERR_INVALID_ARG, "nitems %d outside 1..%d", nitems, b->max_scenes);
-    if (nframes < 1 || nframes > b->max_frames)
-        return fail(GBT_ERR_INVALID_ARG, "nframes %d outside 1..%d", nframes, b->max_frames);
+    gbt_status st = check_items(b, items, nitems, frames, nframes);
+    if (st != GBT_OK) return st;
     if (frames_per_launch < 1 || frames_per_launch > GBT_MAX_FRAMES_PER_SCENE_PASS)
         return fail(GBT_ERR_INVALID_ARG, "frames_per_launch %d outside 1..%d", frames_per_launch,
                     GBT_MAX_FRAMES_PER_SCENE_PASS);
     if (brick < 0 || brick > 3) return fail(GBT_ERR_INVALID_ARG, "brick %d outside 0..3", brick);
     if (ctas_per_sm < 0 || ctas_per_sm > 32) return fail(GBT_ERR_INVALID_ARG, "ctas_per_sm %d outside 0..32", ctas_per_sm);
     const gbt_volume* v0 = items[0].volume;
-    if (!v0) return fail(GBT_ERR_INVALID_ARG, "item 0 has no volume");
     int32_t longest = 0;
     for (int i = 0; i < nitems; ++i) {
         const gbt_batch_item& it = items[i];
-        if (!it.volume) return fail(GBT_ERR_INVALID_ARG, "item %d has no volume", i);
         if (it.volume->cfg.mode != v0->cfg.mode || it.volume->cfg.arith != v0->cfg.arith)
             return fail(GBT_ERR_INVALID_ARG, "item %d: all volumes of a batch need the same mode and arithmetic", i);
-        if (it.nframes < 0 || it.first_frame < 0 || it.first_frame + it.nframes > nframes)
-            return fail(GBT_ERR_INVALID_ARG, "item %d: frames [%d, %d) outside the frame table", i, it.first_frame,
-                        it.first_frame + it.nframes);
         for (int j = 0; j < i; ++j) {
             if (items[j].volume == it.volume) return fail(GBT_ERR_INVALID_ARG, "item %d repeats a volume", i);
             const bool overlap = it.first_frame < items[j].first_frame + items[j].nframes &&
@@ -1033,7 +1113,7 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
         if (it.nframes > longest) longest = it.nframes;
     }
     for (int i = 0; i < nframes; ++i) {
-        gbt_status st = check_frames(frames + i, 1);
+        st = check_frames(frames + i, 1);
         if (st != GBT_OK) return st;
     }
     const int nwin = (longest + frames_per_launch - 1) / frames_per_launch;
@@ -1105,25 +1185,14 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
 
     char* d = static_cast<char*>(b->dev);
     cudaGetLastError();  // a launch reports only its own failure
-    gbt::DepthPyr pyr{nullptr, 0u, 0u};
-    {
-        int32_t mw = 0, mh = 0;
-        uint32_t stride = 0;
-        for (int i = 0; i < nframes; ++i) {
-            mw = std::max(mw, frames[i].width);
-            mh = std::max(mh, frames[i].height);
-        }
-        int64_t work = 0;
-        for (int i = 0; i < nitems; ++i) work += items[i].volume->nvox * items[i].nframes;   // (below 2^32 * 2^24)
-        stride = gbt::pyr_tiles(mw, mh);
-        if (stride && pyramids_pay(work, nframes, (int64_t)mw * mh)) pyr.base = pyr_room(&b->pyr, (size_t)stride * (size_t)nframes, s);
-        if (pyr.base) {
-            pyr.stride = stride;
-            e = gbt::launch_depth_pyramids(
-                reinterpret_cast<const gbt::FrameDesc*>(reinterpret_cast<const gbt::BatchScene*>(d + 256) + b->max_scenes),
-                nframes, mw, mh, pyr, s);
-            if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
-        }
+    const PyrPlan plan = batch_pyramids(items, nitems, frames, nframes);
+    const gbt::DepthPyr pyr = pyr_place(b->pyr, plan);
+    if (pyr.base) {
+        e = gbt::launch_depth_pyramids(
+            reinterpret_cast<const gbt::FrameDesc*>(reinterpret_cast<const gbt::BatchScene*>(d + 256) + b->max_scenes),
+            nframes, plan.width, plan.height, pyr, s);
+        if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
+        count_pyramids(nframes);
     }
     const long long per_sm =
         ctas_per_sm ? ctas_per_sm : gbt::integrate_default_ctas_per_sm(v0->cfg.mode, v0->cfg.arith, 2, brick);

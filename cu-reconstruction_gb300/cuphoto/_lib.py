@@ -31,6 +31,7 @@ MEMORY_DEVICE = 0
 MEMORY_MANAGED = 1
 MAX_FRAMES_PER_PASS = 32
 INJECT_NONE = 0
+COUNT_PYRAMID_LAUNCHES, COUNT_PYRAMID_FRAMES = 0, 1
 INJECT_ALLOC = 1
 INJECT_LAUNCH_ERROR = 2
 INJECT_HOLD_COPY = 3
@@ -138,9 +139,11 @@ SIGNATURES = [
     ("gbt_volume_get_info", C.c_int, [C.c_void_p, C.POINTER(VolumeInfo)]),
     ("gbt_volume_transformation_voxels", C.c_int, [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
     ("gbt_integrate", C.c_int, [C.c_void_p, C.POINTER(Frame), C.c_int32, C.c_void_p]),
+    ("gbt_volume_reserve", C.c_int, [C.c_void_p, C.POINTER(Frame), C.c_int32]),
     ("gbt_integrate_tuned", C.c_int, [C.c_void_p, C.POINTER(Frame), C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     ("gbt_batch_create", C.c_int, [C.c_int32, C.c_int32, C.POINTER(C.c_void_p)]),
     ("gbt_batch_destroy", C.c_int, [C.c_void_p]),
+    ("gbt_batch_reserve", C.c_int, [C.c_void_p, C.POINTER(BatchItem), C.c_int32, C.POINTER(Frame), C.c_int32]),
     ("gbt_integrate_batch", C.c_int, [C.c_void_p, C.POINTER(BatchItem), C.c_int32, C.POINTER(Frame), C.c_int32,
                                       C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     ("gbt_diff_forward", C.c_int, [C.POINTER(DiffCfg), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
@@ -169,6 +172,7 @@ SIGNATURES = [
                                       C.c_void_p]),
     ("gbt_last_error", C.c_char_p, []),
     ("gbt_debug_inject", C.c_int, [C.c_int32, C.c_int64, C.c_int64]),
+    ("gbt_debug_count", C.c_int, [C.c_int32, C.POINTER(C.c_int64)]),
     ("gbt_version", C.c_char_p, []),
 ]
 
@@ -205,6 +209,13 @@ def check(status):
     if status != GBT_OK:
         raise GbtError(status, lib().gbt_last_error().decode())
     return status
+
+
+def debug_count(what):
+    """gbt_debug_count: COUNT_PYRAMID_LAUNCHES or COUNT_PYRAMID_FRAMES so far."""
+    n = C.c_int64()
+    check(lib().gbt_debug_count(what, C.byref(n)))
+    return n.value
 
 
 def device_tensor(t, name):

@@ -83,6 +83,8 @@ class BatchIntegrator:
             n += len(rec)
         fr = np.concatenate(parts) if parts else np.zeros(0, L.frame_dtype())
         self._keep = (items, fr)
+        # room for the depth pyramids (without it: the same result in more time)
+        self._lib.gbt_batch_reserve(self._h, items, len(volumes), fr.ctypes.data_as(C.POINTER(L.Frame)), n)
         L.check(self._lib.gbt_integrate_batch(self._h, items, len(volumes), fr.ctypes.data_as(C.POINTER(L.Frame)), n,
                                               int(frames_per_launch), int(brick), int(ctas_per_sm),
                                               _stream_handle(stream)))

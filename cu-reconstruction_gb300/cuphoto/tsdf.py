@@ -138,8 +138,10 @@ class TSDFVolume:
             self._h = _handle
         else:
             L.check(self._lib.gbt_volume_create(C.byref(cfg.to_c()), _stream_handle(stream), C.byref(self._h)))
+        self._room = None   # the shape of a frame that there is room for
         self._info = L.VolumeInfo()
         L.check(self._lib.gbt_volume_get_info(self._h, C.byref(self._info)))
+        self._voxels = self._info.num_voxels
 
     # -- checkpoint and resume (gbt_volume_save / gbt_volume_load) -------------
     def save(self, path, stream=None):
@@ -220,6 +222,11 @@ class TSDFVolume:
         L.check(self._lib.gbt_volume_check(self._h, _stream_handle(stream)))
 
     # -- integrate -----------------------------------------------------------
+    # Room for the depth pyramids of a pass is asked for (gbt_volume_reserve) where
+    # it has so many voxel-frames that it may use them.  Without the room it gives
+    # the same result in more time, so a failure to provide it is not an error.
+    _PYRAMIDS_FROM = 8 << 20
+
     def integrate(self, color, depth, camera_pose, depth_scale=0.001, stream=None):
         """TSDFVolume::integrate(color, depth, pose) (tsdf_volume.cu:257-290).
 
@@ -234,6 +241,9 @@ class TSDFVolume:
             _log_error("TSDFVolume::integrate() -- depth width/height parameters are zero")
             return False
         f = make_frame(depth, camera_pose, depth_scale)
+        if self._voxels >= self._PYRAMIDS_FROM and depth.shape != self._room:
+            self._lib.gbt_volume_reserve(self._h, f, 1)
+            self._room = depth.shape
         st = self._lib.gbt_integrate(self._h, C.byref(f), 1, _stream_handle(stream))
         if st == L.GBT_ERR_INVALID_ARG:
             _log_error("TSDFVolume::integrate() -- " + self._lib.gbt_last_error().decode())
@@ -250,6 +260,8 @@ class TSDFVolume:
         arr = (L.Frame * n)()
         for i in range(n):
             arr[i] = make_frame(depths[i], poses[i], depth_scale)
+        if n * self._voxels >= self._PYRAMIDS_FROM and brick < 4:
+            self._lib.gbt_volume_reserve(self._h, arr, n)
         L.check(self._lib.gbt_integrate_tuned(self._h, arr, n, int(brick), int(ctas_per_sm), _stream_handle(stream)))
 
     def integrate_sequence(self, depths, poses, frames_per_pass=16, depth_scale=0.001, stream=None, **kw):

@@ -75,7 +75,10 @@ typedef struct {
     float global_offset[3];
     float max_weight;          /* fixed mode: weight clamp; compat: unused (as in the reference) */
     float focal_x, focal_y, cx, cy;
-    uint32_t camera_width, camera_height;   /* informational, as in the reference */
+    /* Informational, as in the reference; frames of any size are accepted.
+     * The volume keeps room for the depth pyramids of GBT_MAX_FRAMES_PER_PASS
+     * frames of this size (see gbt_volume_reserve). */
+    uint32_t camera_width, camera_height;
     float max_cell_size;                   /* unused, as in the reference */
     /* engine options */
     int32_t mode;              /* gbt_mode */
@@ -165,9 +168,21 @@ gbt_status gbt_volume_transformation_voxels(gbt_volume* vol, void* stream, void*
 /* Replaces TSDFVolume::integrate(color, depth, pose) (tsdf_volume.cu:257-290)
  * for `nframes` frames at once: the frames are applied in order, in one
  * pass over the volume (distance and weight read and written once).
- * nframes may be 1..GBT_MAX_FRAMES_PER_PASS.  Asynchronous. */
+ * nframes may be 1..GBT_MAX_FRAMES_PER_PASS.  Asynchronous; allocates
+ * nothing.  Calls of some size (from 8 M voxel-frames on) reduce each frame to a
+ * pyramid of depths first, by which parts of the volume that the frame cannot
+ * update are skipped; a call for which the volume has no room for pyramids goes
+ * without, with the same result in more time. */
 #define GBT_MAX_FRAMES_PER_PASS 32
 gbt_status gbt_integrate(gbt_volume* vol, const gbt_frame* frames, int32_t nframes, void* stream);
+
+/* Makes room for the depth pyramids of a gbt_integrate call with these frames
+ * (their sizes count, the images are not read): at creation a volume has room
+ * for a pass of frames of its configured camera.  8 bytes per 48 pixels a frame,
+ * kept until the volume is destroyed.  Does nothing where there is room, where
+ * pyramids do not pay, or where they would take more than 1 GiB.  May be called
+ * while a stream is being captured. */
+gbt_status gbt_volume_reserve(gbt_volume* vol, const gbt_frame* frames, int32_t nframes);
 
 /* Same as gbt_integrate with an explicit tile shape and grid size, for the
  * autotuner.  brick: 0 = 32x4x4 voxels, 1 = 16x8x4, 2 = 32x2x8, 3 = 64x2x4;
@@ -195,8 +210,12 @@ gbt_status gbt_integrate_tuned(gbt_volume* vol, const gbt_frame* frames, int32_t
  * Results are bit-identical to gbt_integrate on each volume.
  *
  * A gbt_batch owns the device tables of a call (scene and frame descriptors,
- * launch tickets) and a pinned staging copy: a call allocates nothing and
- * records into a CUDA graph as one copy and its launches.  A replay re-reads
+ * launch tickets), a pinned staging copy and room for the depth pyramids of
+ * min(max_frames, 1024) frames of 640x480 (51 KB each): a call allocates nothing
+ * and records into a CUDA graph as one copy and its launches.  Without room for
+ * all of its frames' pyramids it goes without, with the same result in more time;
+ * gbt_batch_reserve makes room for those of a gbt_integrate_batch call with the
+ * same arguments, as gbt_volume_reserve does for a volume.  A replay re-reads
  * the staging area as the last call on the batch object left it, so a graph
  * should hold one call per batch object.  One host thread per batch object.
  * brick (0..3) and ctas_per_sm as for gbt_integrate_tuned. */
@@ -209,6 +228,8 @@ typedef struct {
 } gbt_batch_item;
 gbt_status gbt_batch_create(int32_t max_scenes, int32_t max_frames, gbt_batch** out);
 gbt_status gbt_batch_destroy(gbt_batch* batch);
+gbt_status gbt_batch_reserve(gbt_batch* batch, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
+                             int32_t nframes);
 gbt_status gbt_integrate_batch(gbt_batch* batch, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
                                int32_t nframes, int32_t frames_per_launch, int32_t brick, int32_t ctas_per_sm,
                                void* stream);
@@ -450,6 +471,14 @@ enum {
     GBT_INJECT_HOLD_COPY = 3
 };
 gbt_status gbt_debug_inject(int32_t what, int64_t skip, int64_t count);
+
+/* Counts since the library was loaded, over all threads, for tests and
+ * benchmarks: launches that built depth pyramids, and frames that got one. */
+enum {
+    GBT_COUNT_PYRAMID_LAUNCHES = 0,
+    GBT_COUNT_PYRAMID_FRAMES = 1
+};
+gbt_status gbt_debug_count(int32_t what, int64_t* value);
 
 /* Engine version string. */
 const char* gbt_version(void);

@@ -1,0 +1,220 @@
+"""Depth pyramids and the room for them.  The integrate calls of the C ABI take
+the room that is there or go without, and allocate nothing; the reserve calls
+(which the Python and C++ layers make) provide it, while streams are being
+captured too.  With and without pyramids the volume is the same."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from cuphoto import TSDFVolume, _lib as L
+from cuphoto import synthetic as S
+from cuphoto.batch import BatchIntegrator
+from cuphoto.tsdf import make_frame
+
+from helpers import dev_depth
+from test_gpu_depth_cull import config, frames, volume_bits
+
+pytestmark = pytest.mark.gpu
+
+GRID = (96, 80, 72)   # 8.8 M voxel-frames with 16 frames
+
+
+def counted(call):
+    """(launches, frames) of depth pyramids in call()."""
+    c = [L.debug_count(k) for k in (L.COUNT_PYRAMID_LAUNCHES, L.COUNT_PYRAMID_FRAMES)]
+    call()
+    return tuple(L.debug_count(k) - c[k] for k in (L.COUNT_PYRAMID_LAUNCHES, L.COUNT_PYRAMID_FRAMES))
+
+
+def plain_integrate(vol, dd, poses, stream=None):
+    """gbt_integrate without a reserve call."""
+    arr = (L.Frame * len(dd))(*[make_frame(d, p) for d, p in zip(dd, poses)])
+    L.check(L.lib().gbt_integrate(vol.handle, arr, len(dd), stream.cuda_stream if stream is not None else None))
+
+
+def plain_batch(batch, vols, dds, poses, stream=None):
+    """gbt_integrate_batch without a reserve call."""
+    arr, items = [], (L.BatchItem * len(vols))()
+    for k, (v, dd, ps) in enumerate(zip(vols, dds, poses)):
+        items[k] = L.BatchItem(v.handle.value, len(arr), len(dd))
+        arr += [make_frame(d, p) for d, p in zip(dd, ps)]
+    L.check(L.lib().gbt_integrate_batch(batch._h, items, len(vols), (L.Frame * len(arr))(*arr), len(arr), 128, 0, 0,
+                                        stream.cuda_stream if stream is not None else None))
+
+
+@pytest.fixture(scope="module")
+def half():
+    return frames("frontal", "u16", 4)
+
+
+@pytest.fixture(scope="module")
+def hd():
+    cam = S.Camera.hd()
+    seq = S.make_sequence(16, scene_id=2, camera=cam, trajectory="frontal")
+    return list(seq.depth_u16), seq.poses, cam
+
+
+def want(gpu, tc, dd, poses):
+    vol = TSDFVolume(tc)
+    vol.integrate_frames(dd, poses, brick=4)   # without pyramids
+    return volume_bits(gpu, vol)
+
+
+def same(gpu, vol, bits):
+    D, W = volume_bits(gpu, vol)
+    return np.array_equal(D, bits[0]) and np.array_equal(W, bits[1])
+
+
+@pytest.mark.parametrize("mode,arith", [("compat", "ieee"), ("fixed", "ieee"), ("compat", "reference")])
+@pytest.mark.parametrize("camera", [(0, 0), (64, 48), (160, 120)])
+def test_calls_without_room_go_without(gpu, half, camera, mode, arith):
+    depths, poses, cam = half
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam, mode=mode, arith=arith, camera_width=camera[0], camera_height=camera[1])
+    bits = want(gpu, tc, dd, poses)
+    vol = TSDFVolume(tc)
+    warm = TSDFVolume(tc)
+    for call in (plain_integrate, lambda v, *a: v.integrate_frames(*a)):   # (kernels are loaded by their first launch)
+        call(warm, dd, poses)
+    gpu.cuda.synchronize()
+    free = gpu.cuda.mem_get_info()[0]
+    assert counted(lambda: plain_integrate(vol, dd, poses)) == (0, 0)
+    gpu.cuda.synchronize()
+    assert gpu.cuda.mem_get_info()[0] == free
+    assert same(gpu, vol, bits)
+    vol.reset()
+    assert counted(lambda: vol.integrate_frames(dd, poses)) == (1, 16)   # the Python layer reserves
+    assert same(gpu, vol, bits)
+    vol.reset()
+    assert counted(lambda: plain_integrate(vol, dd, poses)) == (1, 16)   # and what it reserved stays
+    assert same(gpu, vol, bits)
+
+
+def test_batched_calls_without_room_go_without(gpu, hd):
+    depths, poses, cam = hd
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam, mode="fixed")
+    bits = want(gpu, tc, dd, poses)
+    vol = TSDFVolume(tc)
+    plain_batch(BatchIntegrator(1, 16), [vol], [dd], [poses])   # (kernels are loaded by their first launch)
+    vol.reset()
+    batch = BatchIntegrator(1, 16)
+    gpu.cuda.synchronize()
+    free = gpu.cuda.mem_get_info()[0]
+    assert counted(lambda: plain_batch(batch, [vol], [dd], [poses])) == (0, 0)
+    gpu.cuda.synchronize()
+    assert gpu.cuda.mem_get_info()[0] == free
+    assert same(gpu, vol, bits)
+    vol.reset()
+    assert counted(lambda: batch.integrate([vol], [dd], [poses])) == (1, 16)
+    assert same(gpu, vol, bits)
+
+
+@pytest.mark.parametrize("reserve", [False, True])
+@pytest.mark.parametrize("batched", [False, True])
+def test_graphs_without_pyramids_and_with_an_outgrown_buffer(gpu, half, hd, batched, reserve):
+    """Captured on objects that have too little room: without pyramids, or after a
+    reserve call under capture.  Replayed as captured, and once more after a
+    larger call has moved the buffer."""
+    depths, poses, cam = hd if batched else half
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam, camera_width=64, camera_height=48)
+    bits = want(gpu, tc, dd, poses)
+    vol, other = TSDFVolume(tc), TSDFVolume(tc)
+    batch, larger = BatchIntegrator(1, 16), BatchIntegrator(1, 16)
+    s, g = gpu.cuda.Stream(), gpu.cuda.CUDAGraph()
+
+    def record():
+        with gpu.cuda.graph(g, stream=s):
+            if batched and reserve:
+                batch.integrate([vol], [dd], [poses], stream=s)
+            elif batched:
+                plain_batch(batch, [vol], [dd], [poses], s)
+            elif reserve:
+                vol.integrate_frames(dd, poses, stream=s)
+            else:
+                plain_integrate(vol, dd, poses, s)
+
+    assert counted(record) == ((1, 16) if reserve else (0, 0))
+    g.replay()
+    assert same(gpu, vol, bits)
+    if batched:   # (a graph reads the staging area of its batch's last call: another batch grows)
+        larger.integrate([other], [dd], [poses])
+    else:
+        vol.integrate_frames(dd + dd, list(poses) + list(poses))
+    vol.reset()
+    gpu.cuda.synchronize()
+    g.replay()
+    assert same(gpu, vol, bits)
+
+
+def test_without_memory_for_pyramids(gpu, half):
+    depths, poses, cam = half
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam, camera_width=0, camera_height=0)
+    bits = want(gpu, tc, dd, poses)
+    vol = TSDFVolume(tc)
+    try:
+        L.lib().gbt_debug_inject(L.INJECT_ALLOC, 0, 1)
+        assert counted(lambda: vol.integrate_frames(dd, poses)) == (0, 0)
+    finally:
+        L.lib().gbt_debug_inject(L.INJECT_NONE, 0, 0)
+    assert same(gpu, vol, bits)
+    arr = (L.Frame * 16)(*[make_frame(d, p) for d, p in zip(dd, poses)])
+    assert L.lib().gbt_volume_reserve(vol.handle, arr, 16) == L.GBT_OK
+    vol.reset()
+    assert counted(lambda: vol.integrate_frames(dd, poses)) == (1, 16)
+    assert same(gpu, vol, bits)
+
+
+def test_growth_does_not_end_another_thread_s_capture(gpu, half):
+    """A capture in global mode forbids other threads' allocations, unless they
+    are marked as harmless to it."""
+    depths, poses, cam = half
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam, camera_width=64, camera_height=48)
+    bits = want(gpu, tc, dd, poses)
+    a, b = TSDFVolume(tc), TSDFVolume(tc)
+    s, t, g = gpu.cuda.Stream(), gpu.cuda.Stream(), gpu.cuda.CUDAGraph()
+    failed = []
+
+    def work():
+        try:
+            b.integrate_frames(dd, poses, stream=t)
+        except Exception as e:
+            failed.append(e)
+
+    gpu.cuda.synchronize()
+    with gpu.cuda.graph(g, stream=s, capture_error_mode="global"):
+        a.integrate_frames(dd, poses, stream=s)
+        th = threading.Thread(target=work)
+        th.start()
+        th.join()
+    assert not failed
+    g.replay()
+    assert same(gpu, a, bits) and same(gpu, b, bits)
+
+
+def test_reserve_calls_check_their_arguments(gpu, half):
+    depths, poses, cam = half
+    vol = TSDFVolume(config("frontal", (16, 16, 16), cam))
+    f = make_frame(dev_depth(gpu, depths[0]), poses[0])
+    lib = L.lib()
+    assert lib.gbt_volume_reserve(None, C.byref(f), 1) == L.GBT_ERR_INVALID_ARG
+    for n in (0, 33):
+        assert lib.gbt_volume_reserve(vol.handle, (L.Frame * 33)(f), n) == L.GBT_ERR_INVALID_ARG
+    bad = L.Frame()
+    assert lib.gbt_volume_reserve(vol.handle, C.byref(bad), 1) == L.GBT_ERR_INVALID_ARG
+    batch = BatchIntegrator(1, 2)
+    ok = (L.Frame * 2)(f, f)
+    for items in ([(None, 0, 1)], [(vol.handle.value, 0, 3)], [(vol.handle.value, -1, 1)], [(vol.handle.value, 0, 1)] * 2):
+        it = (L.BatchItem * len(items))(*[L.BatchItem(*i) for i in items])
+        assert lib.gbt_batch_reserve(batch._h, it, len(items), ok, 2) == L.GBT_ERR_INVALID_ARG
+    one = (L.BatchItem * 1)(L.BatchItem(vol.handle.value, 0, 2))
+    assert lib.gbt_batch_reserve(batch._h, one, 1, ok, 3) == L.GBT_ERR_INVALID_ARG
+    assert lib.gbt_batch_reserve(batch._h, one, 1, ok, 2) == L.GBT_OK
+    n = C.c_int64()
+    assert lib.gbt_debug_count(7, C.byref(n)) == L.GBT_ERR_INVALID_ARG
+    assert lib.gbt_debug_count(0, None) == L.GBT_ERR_INVALID_ARG
