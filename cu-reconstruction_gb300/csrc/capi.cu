@@ -88,9 +88,9 @@ namespace {
 // Launches of depth pyramids and frames that got one (gbt_debug_count).
 std::atomic<int64_t> g_pyramid_launches{0}, g_pyramid_frames{0};
 
-// A volume's or batch's buffer for depth pyramids: at first the end of its own
-// device allocation, a larger one of its own once the caller asks for it
-// (pyr_reserve; the integrate calls take what is there).  Buffers that were
+// A volume's or batch's buffer for depth pyramids: one made with it, if there is
+// memory for it, and a larger one once the caller asks for it (pyr_reserve; the
+// integrate calls take what is there).  Buffers that were
 // outgrown stay until the owner goes, since a captured graph may read them (they
 // add up to less than the last one, which is at least twice as large as the one
 // before, or to kPyrMaxBytes before a last one of that size).
@@ -142,6 +142,20 @@ gbt_status pyr_reserve(PyrBuffer* b, const PyrPlan& p) {
     b->data = static_cast<float2*>(p0);
     b->tiles = want;
     return GBT_OK;
+}
+
+// The room of a new volume or batch.  (Pyramids are optional, so a failure to
+// allocate it is none.)
+void pyr_create(PyrBuffer* b, size_t tiles) {
+    if (tiles == 0) return;
+    void* p = nullptr;
+    if (dev_alloc(&p, tiles * sizeof(float2)) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    b->own[b->nown++] = p;
+    b->data = static_cast<float2*>(p);
+    b->tiles = tiles;
 }
 
 void pyr_free(PyrBuffer* b) {
@@ -267,6 +281,18 @@ bool layer_runs_pay(const gbt_volume* v, int32_t n) {
 // for one frame the line is at twelve million.
 bool pyramids_pay(int64_t voxel_frames, int64_t frames, int64_t pixels) {
     return voxel_frames >= (int64_t)(frames == 1 ? 12 : 8) << 20 && voxel_frames >= frames * (pixels / 2);
+}
+
+// Tiles of room that a new volume makes: for the longest pass of frames of its
+// configured camera (1.6 MB for 640x480, 4.7 MB for 1280x720), as far as a quarter
+// of the grid's own bytes goes, and where such a pass can use them at all.
+size_t first_room(const gbt_volume_cfg& c, int64_t nvox) {
+    constexpr uint32_t kMaxSide = 1u << 16;
+    if (c.camera_width == 0 || c.camera_height == 0 || c.camera_width > kMaxSide || c.camera_height > kMaxSide) return 0;
+    const size_t frame = gbt::pyr_tiles((int32_t)c.camera_width, (int32_t)c.camera_height);
+    const size_t quarter = (size_t)nvox * 2 * sizeof(float) / 4 / sizeof(float2);
+    const int64_t n = std::min((int64_t)GBT_MAX_FRAMES_PER_PASS, (int64_t)(quarter / frame));
+    return n > 0 && pyramids_pay(nvox * n, n, (int64_t)c.camera_width * c.camera_height) ? (size_t)n * frame : 0;
 }
 
 // Raises d->clear, how near the camera plane boxes of voxels are tested as boxes, to
@@ -494,12 +520,9 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
     d.cy = c.cy;
 
     const size_t bytes = (size_t)nvox * sizeof(float);
-    // the status word sits 256-byte aligned after the distances, then the depth
-    // pyramids of one pass of frames of the configured camera
+    // the status word sits 256-byte aligned after the distances
     const size_t status_at = (bytes + 255) / 256 * 256;
-    if (c.camera_width > 0 && c.camera_height > 0 && c.camera_width <= 4096 && c.camera_height <= 4096)
-        v->pyr.tiles = (size_t)gbt::pyr_tiles(c.camera_width, c.camera_height) * GBT_MAX_FRAMES_PER_PASS;
-    const size_t d_bytes = status_at + 256 + v->pyr.tiles * sizeof(float2);
+    const size_t d_bytes = status_at + 256;
     cudaError_t e;
     if (v->managed) {
         e = dev_alloc(reinterpret_cast<void**>(&d.D), d_bytes, true);
@@ -508,10 +531,7 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
         e = dev_alloc(reinterpret_cast<void**>(&d.D), d_bytes);
         if (e == cudaSuccess) e = dev_alloc(reinterpret_cast<void**>(&d.W), bytes);
     }
-    if (e == cudaSuccess) {
-        v->status = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(d.D) + status_at);
-        v->pyr.data = reinterpret_cast<float2*>(reinterpret_cast<char*>(d.D) + status_at + 256);
-    }
+    if (e == cudaSuccess) v->status = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(d.D) + status_at);
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (d.D) cudaFree(d.D);
@@ -519,6 +539,7 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
         delete v;
         return fail(GBT_ERR_ALLOC, "allocating %zu bytes for the volume: %s", 2 * bytes, cudaGetErrorString(e));
     }
+    pyr_create(&v->pyr, first_room(c, nvox));
     gbt_status st = gbt_volume_reset(v, stream);
     if (st == GBT_OK) {
         e = cudaStreamSynchronize(as_stream(stream));
@@ -527,6 +548,7 @@ gbt_status gbt_volume_create(const gbt_volume_cfg* cfg, void* stream, gbt_volume
     if (st != GBT_OK) {
         cudaFree(d.D);
         cudaFree(d.W);
+        pyr_free(&v->pyr);
         delete v;
         return st;
     }
@@ -1044,12 +1066,8 @@ gbt_status gbt_batch_create(int32_t max_scenes, int32_t max_frames, gbt_batch** 
     b->max_scenes = max_scenes;
     b->max_frames = max_frames;
     b->bytes = batch_bytes(max_scenes, max_frames);
-    // the device tables are followed by the depth pyramids of up to 1024 frames of 640x480 (52 MB)
-    const size_t pyr_at = (b->bytes + 255) / 256 * 256;
-    b->pyr.tiles = (size_t)gbt::pyr_tiles(640, 480) * (size_t)std::min(max_frames, 1024);
     cudaError_t e = pinned_alloc(&b->host, b->bytes);
-    if (e == cudaSuccess) e = dev_alloc(&b->dev, pyr_at + b->pyr.tiles * sizeof(float2));
-    if (e == cudaSuccess) b->pyr.data = reinterpret_cast<float2*>(static_cast<char*>(b->dev) + pyr_at);
+    if (e == cudaSuccess) e = dev_alloc(&b->dev, b->bytes);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -1058,6 +1076,7 @@ gbt_status gbt_batch_create(int32_t max_scenes, int32_t max_frames, gbt_batch** 
         delete b;
         return fail(GBT_ERR_ALLOC, "batch tables: %s", cudaGetErrorString(e));
     }
+    pyr_create(&b->pyr, (size_t)gbt::pyr_tiles(640, 480) * (size_t)std::min(max_frames, 1024));   // (52 MB at most)
     *out = b;
     return GBT_OK;
 }

@@ -76,8 +76,9 @@ typedef struct {
     float max_weight;          /* fixed mode: weight clamp; compat: unused (as in the reference) */
     float focal_x, focal_y, cx, cy;
     /* Informational, as in the reference; frames of any size are accepted.
-     * The volume keeps room for the depth pyramids of GBT_MAX_FRAMES_PER_PASS
-     * frames of this size (see gbt_volume_reserve). */
+     * Where the grid is large enough to use them, the volume keeps room for the
+     * depth pyramids of GBT_MAX_FRAMES_PER_PASS frames of this size, of up to a
+     * quarter of the grid's bytes (see gbt_volume_reserve). */
     uint32_t camera_width, camera_height;
     float max_cell_size;                   /* unused, as in the reference */
     /* engine options */
@@ -177,8 +178,8 @@ gbt_status gbt_volume_transformation_voxels(gbt_volume* vol, void* stream, void*
 gbt_status gbt_integrate(gbt_volume* vol, const gbt_frame* frames, int32_t nframes, void* stream);
 
 /* Makes room for the depth pyramids of a gbt_integrate call with these frames
- * (their sizes count, the images are not read): at creation a volume has room
- * for a pass of frames of its configured camera.  8 bytes per 48 pixels a frame,
+ * (their sizes count, the images are not read): a volume is created with room
+ * for frames of its configured camera, if there is memory for it.  8 bytes per 48 pixels a frame,
  * kept until the volume is destroyed.  Does nothing where there is room, where
  * pyramids do not pay, or where they would take more than 1 GiB.  May be called
  * while a stream is being captured. */
@@ -210,14 +211,14 @@ gbt_status gbt_integrate_tuned(gbt_volume* vol, const gbt_frame* frames, int32_t
  * Results are bit-identical to gbt_integrate on each volume.
  *
  * A gbt_batch owns the device tables of a call (scene and frame descriptors,
- * launch tickets), a pinned staging copy and room for the depth pyramids of
- * min(max_frames, 1024) frames of 640x480 (51 KB each): a call allocates nothing
- * and records into a CUDA graph as one copy and its launches.  Without room for
- * all of its frames' pyramids it goes without, with the same result in more time;
- * gbt_batch_reserve makes room for those of a gbt_integrate_batch call with the
- * same arguments, as gbt_volume_reserve does for a volume.  A replay re-reads
- * the staging area as the last call on the batch object left it, so a graph
- * should hold one call per batch object.  One host thread per batch object.
+ * launch tickets), a pinned staging copy and, if there is memory for it, room for
+ * the depth pyramids of min(max_frames, 1024) frames of 640x480 (51 KB each): a
+ * call allocates nothing and records into a CUDA graph as one copy and its
+ * launches.  Without room for all of its frames' pyramids it goes without, with
+ * the same result in more time; gbt_batch_reserve makes room for those of a
+ * gbt_integrate_batch call with the same arguments, as gbt_volume_reserve does
+ * for a volume.  A replay re-reads the staging area as the last call on the batch
+ * object left it, so a graph should hold one call per batch object.  One host thread per batch object.
  * brick (0..3) and ctas_per_sm as for gbt_integrate_tuned. */
 #define GBT_MAX_FRAMES_PER_SCENE_PASS 128
 typedef struct gbt_batch gbt_batch;

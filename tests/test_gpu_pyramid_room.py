@@ -218,3 +218,51 @@ def test_reserve_calls_check_their_arguments(gpu, half):
     n = C.c_int64()
     assert lib.gbt_debug_count(7, C.byref(n)) == L.GBT_ERR_INVALID_ARG
     assert lib.gbt_debug_count(0, None) == L.GBT_ERR_INVALID_ARG
+
+
+def test_creation_without_memory_for_pyramids(gpu, half, hd):
+    """The room is optional: its allocation, the last of a volume's or batch's,
+    may fail."""
+    depths, poses, cam = half
+    dd = [dev_depth(gpu, d) for d in depths]
+    tc = config("frontal", GRID, cam)
+    bits = want(gpu, tc, dd, poses)
+    made = []
+    try:
+        for create in (lambda: TSDFVolume(tc), lambda: BatchIntegrator(1, 16)):
+            L.lib().gbt_debug_inject(L.INJECT_ALLOC, 2, 1)
+            made.append(create())
+    finally:
+        L.lib().gbt_debug_inject(L.INJECT_NONE, 0, 0)
+    vol, batch = made
+    assert counted(lambda: plain_integrate(vol, dd, poses)) == (0, 0)
+    assert same(gpu, vol, bits)
+    vol.reset()
+    assert counted(lambda: plain_batch(batch, [vol], [dd], [poses])) == (0, 0)
+    assert same(gpu, vol, bits)
+    vol.reset()
+    assert counted(lambda: batch.integrate([vol], [dd], [poses])) == (1, 16)
+    assert same(gpu, vol, bits)
+
+
+@pytest.mark.parametrize("grid,camera,frames_with_room", [
+    ((64, 64, 64), (640, 480), 0),        # they pay from 32 frames; a quarter of the grid's 2 MB has room for 10
+    ((96, 80, 72), (640, 480), 21),       # a quarter of its bytes
+    ((160, 160, 160), (640, 480), 32),
+    ((160, 160, 160), (1280, 720), 32),
+    ((64, 64, 64), (1280, 720), 0),       # more than two pixels a voxel: pyramids do not pay
+    ((48, 48, 48), (640, 480), 0),        # below 8 M voxel-frames in any pass
+    ((64, 64, 64), (4096, 4096), 0)])
+def test_room_at_creation_is_that_of_the_grid(gpu, grid, camera, frames_with_room):
+    """How many frames of the configured camera one pass can have pyramids of,
+    without a reserve call; larger passes go without."""
+    w, h = camera
+    vol = TSDFVolume(config("circle", grid, S.Camera.half(), camera_width=w, camera_height=h))
+    img = gpu.zeros((h, w), dtype=gpu.int16, device="cuda")
+    pose = S.circle_poses(8)[0]
+    most = 0
+    for n in range(1, 33):
+        c = counted(lambda: plain_integrate(vol, [img] * n, [pose] * n))
+        if c == (1, n):
+            most = n
+    assert most == frames_with_room
