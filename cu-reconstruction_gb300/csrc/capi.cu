@@ -102,23 +102,26 @@ struct PyrBuffer {
 };
 constexpr size_t kPyrMaxBytes = (size_t)1 << 30;   // 20,000 frames of 640x480
 
-// The pyramids of a call: of frames of up to width x height, `frames` of them.
+// The pyramids of a call: of frames [first, first + frames) of its table, of up to
+// width x height.
 struct PyrPlan {
     int32_t width, height;
     uint32_t stride;   // tiles per frame; 0: pyramids do not pay
-    uint32_t frames;
+    uint32_t first, frames;
+    uint32_t used;     // frames of the range that are integrated; the others stay unread
 };
 
-// The plan's pyramids in `b`, none if there is no room for all of them.
+// The plan's pyramids in `b`, that of frame `first` first; none if there is no room
+// for all of them.
 gbt::DepthPyr pyr_place(const PyrBuffer& b, const PyrPlan& p) {
     gbt::DepthPyr d{nullptr, p.stride, 0u};
     if (p.stride && (size_t)p.stride * p.frames <= b.tiles) d.base = b.data;
     return d;
 }
 
-void count_pyramids(int64_t frames) {
-    g_pyramid_launches.fetch_add((frames + 65534) / 65535, std::memory_order_relaxed);
-    g_pyramid_frames.fetch_add(frames, std::memory_order_relaxed);
+void count_pyramids(const PyrPlan& p) {
+    g_pyramid_launches.fetch_add((p.frames + 65534u) / 65535u, std::memory_order_relaxed);
+    g_pyramid_frames.fetch_add(p.used, std::memory_order_relaxed);
 }
 
 // Room for the plan's pyramids, if they are not too large.
@@ -331,7 +334,7 @@ void add_clear(const gbt_volume_cfg& c, const gbt::FrameDesc& f, gbt::VolDesc* d
 
 // The depth pyramids of a pass of checked frames.
 PyrPlan pass_pyramids(const gbt_volume* v, const gbt_frame* frames, int32_t n) {
-    PyrPlan p{0, 0, 0u, (uint32_t)n};
+    PyrPlan p{0, 0, 0u, 0u, (uint32_t)n, (uint32_t)n};
     for (int i = 0; i < n; ++i) {
         p.width = std::max(p.width, frames[i].width);
         p.height = std::max(p.height, frames[i].height);
@@ -814,7 +817,7 @@ gbt_status gbt_integrate_tuned(gbt_volume* v, const gbt_frame* frames, int32_t n
         if (a.pyr.base) {
             e = gbt::launch_depth_pyramids(a, p.width, p.height, as_stream(stream));
             if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
-            count_pyramids(nframes);
+            count_pyramids(p);
         }
     }
     if (brick == 8) {
@@ -1039,16 +1042,33 @@ gbt_status check_items(const gbt_batch* b, const gbt_batch_item* items, int32_t 
     return GBT_OK;
 }
 
-// The depth pyramids of a batched call whose items have been checked.
-PyrPlan batch_pyramids(const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames, int32_t nframes) {
-    PyrPlan p{0, 0, 0u, (uint32_t)nframes};
-    for (int i = 0; i < nframes; ++i) {
+// The depth pyramids of a batched call whose items have been checked, and which
+// frames its items take: a caller may keep one long table, of which the images of
+// other frames need not be there.
+PyrPlan batch_pyramids(const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames, int32_t nframes,
+                       std::vector<char>* used) {
+    PyrPlan p{0, 0, 0u, 0u, 0u, 0u};
+    used->assign((size_t)nframes, 0);
+    int32_t first = nframes, end = 0;
+    int64_t work = 0;
+    for (int i = 0; i < nitems; ++i) {
+        const gbt_batch_item& it = items[i];
+        work += it.volume->nvox * it.nframes;   // (below 2^32 * 2^24)
+        if (it.nframes == 0) continue;
+        first = std::min(first, it.first_frame);
+        end = std::max(end, it.first_frame + it.nframes);
+        std::fill_n(used->begin() + it.first_frame, it.nframes, 1);
+    }
+    for (int i = first; i < end; ++i) {
+        if (!(*used)[i]) continue;
+        ++p.used;
         p.width = std::max(p.width, frames[i].width);
         p.height = std::max(p.height, frames[i].height);
     }
-    int64_t work = 0;
-    for (int i = 0; i < nitems; ++i) work += items[i].volume->nvox * items[i].nframes;   // (below 2^32 * 2^24)
-    if (pyramids_pay(work, nframes, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
+    if (p.used == 0) return p;
+    p.first = (uint32_t)first;
+    p.frames = (uint32_t)(end - first);
+    if (pyramids_pay(work, p.used, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
     return p;
 }
 
@@ -1099,7 +1119,8 @@ gbt_status gbt_batch_reserve(gbt_batch* b, const gbt_batch_item* items, int32_t 
     for (int i = 0; i < nframes; ++i)
         if (frames[i].width <= 0 || frames[i].height <= 0)
             return fail(GBT_ERR_INVALID_ARG, "frame %d: depth width/height are zero", i);
-    return pyr_reserve(&b->pyr, batch_pyramids(items, nitems, frames, nframes));
+    std::vector<char> used;
+    return pyr_reserve(&b->pyr, batch_pyramids(items, nitems, frames, nframes, &used));
 }
 
 gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_t nitems, const gbt_frame* frames,
@@ -1150,10 +1171,13 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
     gbt::brick_extent(brick, &bx, &by, &bz);
     gbt::BatchScene* hs = reinterpret_cast<gbt::BatchScene*>(static_cast<char*>(b->host) + 256);
     gbt::FrameDesc* hf = reinterpret_cast<gbt::FrameDesc*>(hs + b->max_scenes);
+    std::vector<char> used_frames;
+    const PyrPlan plan = batch_pyramids(items, nitems, frames, nframes, &used_frames);
     for (int i = 0; i < nframes; ++i) {
         const gbt_frame& f = frames[i];
         gbt::FrameDesc& fd = hf[i];
         std::memset(&fd, 0, sizeof(fd));
+        if (!used_frames[i]) continue;   // an image of no pixels
         fd.depth = f.depth;
         fd.pitch = (int64_t)f.pitch_bytes;
         fd.width = f.width;
@@ -1204,14 +1228,15 @@ gbt_status gbt_integrate_batch(gbt_batch* b, const gbt_batch_item* items, int32_
 
     char* d = static_cast<char*>(b->dev);
     cudaGetLastError();  // a launch reports only its own failure
-    const PyrPlan plan = batch_pyramids(items, nitems, frames, nframes);
-    const gbt::DepthPyr pyr = pyr_place(b->pyr, plan);
+    gbt::DepthPyr pyr = pyr_place(b->pyr, plan);
     if (pyr.base) {
         e = gbt::launch_depth_pyramids(
-            reinterpret_cast<const gbt::FrameDesc*>(reinterpret_cast<const gbt::BatchScene*>(d + 256) + b->max_scenes),
-            nframes, plan.width, plan.height, pyr, s);
+            reinterpret_cast<const gbt::FrameDesc*>(reinterpret_cast<const gbt::BatchScene*>(d + 256) + b->max_scenes) +
+                plan.first,
+            (int)plan.frames, plan.width, plan.height, pyr, s);
         if (e != cudaSuccess) return cuda_fail(e, "depth pyramids");
-        count_pyramids(nframes);
+        count_pyramids(plan);
+        pyr.base -= (size_t)plan.first * plan.stride;   // (the kernels look up by a frame's number in the table)
     }
     const long long per_sm =
         ctas_per_sm ? ctas_per_sm : gbt::integrate_default_ctas_per_sm(v0->cfg.mode, v0->cfg.arith, 2, brick);

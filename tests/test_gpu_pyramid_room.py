@@ -266,3 +266,26 @@ def test_room_at_creation_is_that_of_the_grid(gpu, grid, camera, frames_with_roo
         if c == (1, n):
             most = n
     assert most == frames_with_room
+
+
+def test_frames_that_no_item_takes_get_no_pyramid(gpu, half):
+    """A long table of which the items take a few ranges."""
+    depths, poses, cam = half
+    dd = [dev_depth(gpu, d) for d in depths]
+    n = len(dd)
+    tc = config("frontal", GRID, cam, mode="fixed")
+    vols = [TSDFVolume(tc) for _ in range(3)]
+    ranges = [(7, 9), (20, 5), (24, 6)]         # frames 7-15, 20-24 and 24-29 of 40
+    table = [make_frame(dd[k % n], poses[k % n]) for k in range(40)]
+    for k in range(40):
+        if not any(a <= k < a + c for a, c in ranges):
+            table[k].width = table[k].height = 1   # small images: none of them is read
+            table[k].pitch_bytes = 2
+    items = (L.BatchItem * 3)(*[L.BatchItem(v.handle.value, a, c) for v, (a, c) in zip(vols, ranges)])
+    batch = BatchIntegrator(3, 40)
+    st = counted(lambda: L.check(L.lib().gbt_integrate_batch(batch._h, items, 3, (L.Frame * 40)(*table), 40, 128, 0, 0,
+                                                             None)))
+    assert st == (1, 9 + 5 + 6 - 1)
+    for v, (a, c) in zip(vols, ranges):
+        k = [i % n for i in range(a, a + c)]
+        assert same(gpu, v, want(gpu, tc, [dd[i] for i in k], [poses[i] for i in k]))
