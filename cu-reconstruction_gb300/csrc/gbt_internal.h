@@ -101,7 +101,10 @@ struct DepthPyr {
     uint32_t pad0;
     __host__ __device__ const float2* of(int frame) const { return base ? base + (size_t)frame * stride : nullptr; }
 };
+// Tiles of an image's pyramid, 0 for images that go without one: with a side of more
+// than 65535 blocks of 128 pixels, the most that a launch has along y.
 inline uint32_t pyr_tiles(int32_t width, int32_t height) {
+    if (width > 65535 * 128 || height > 65535 * 128) return 0u;
     uint64_t n = 0;
     uint32_t w = ((uint32_t)width + 7u) >> 3, h = ((uint32_t)height + 7u) >> 3;
     for (int l = 0; l < kPyrLevels; ++l) {
@@ -109,7 +112,7 @@ inline uint32_t pyr_tiles(int32_t width, int32_t height) {
         w = (w + 1u) >> 1;
         h = (h + 1u) >> 1;
     }
-    return n > 0xffffffffull ? 0u : (uint32_t)n;   // (an image of more than 2^37 pixels: none)
+    return (uint32_t)n;   // (below 2^27: an image has at most 2^32 pixels)
 }
 
 struct IntegrateArgs {

@@ -8,7 +8,7 @@ import threading
 import numpy as np
 import pytest
 
-from cuphoto import TSDFVolume, _lib as L
+from cuphoto import TSDFVolume, TSDFVolumeConfig, _lib as L
 from cuphoto import synthetic as S
 from cuphoto.batch import BatchIntegrator
 from cuphoto.tsdf import make_frame
@@ -289,3 +289,24 @@ def test_frames_that_no_item_takes_get_no_pyramid(gpu, half):
     for v, (a, c) in zip(vols, ranges):
         k = [i % n for i in range(a, a + c)]
         assert same(gpu, v, want(gpu, tc, [dd[i] for i in k], [poses[i] for i in k]))
+
+
+@pytest.mark.parametrize("height,with_pyramid", [(65535 * 128, 1), (65535 * 128 + 1, 0)])
+def test_images_taller_than_a_grid_of_blocks(gpu, height, with_pyramid):
+    """An image of two columns and more rows than one launch's blocks cover is
+    integrated without a pyramid, by single passes and by the batch."""
+    n, w = 240, 2
+    tc = TSDFVolumeConfig(voxel_grid_size=(n, n, n), physical_size=(1.0, 1.0, 1.0), global_offset=(-0.5, -0.5, 0.5),
+                          focal_x=1.5, focal_y=200.0, cx=0.5, cy=150.0, camera_width=w, camera_height=300, mode="fixed")
+    img = gpu.full((height, w), 1000, dtype=gpu.int16, device="cuda")
+    img[100:130] = 0
+    pose = np.array([1.0, 0, 0, 0, 0, 0, 0])
+    bits = want(gpu, tc, [img], [pose])
+    assert (bits[1] > 0).mean() > 0.1
+    vol = TSDFVolume(tc)
+    assert counted(lambda: vol.integrate(img, img, pose)) == (with_pyramid, with_pyramid)
+    assert same(gpu, vol, bits)
+    vol.reset()
+    batch = BatchIntegrator(1, 1)
+    assert counted(lambda: batch.integrate([vol], [[img]], [[pose]])) == (with_pyramid, with_pyramid)
+    assert same(gpu, vol, bits)
