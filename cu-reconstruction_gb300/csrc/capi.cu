@@ -1035,9 +1035,9 @@ gbt_status check_items(const gbt_batch* b, const gbt_batch_item* items, int32_t 
     for (int i = 0; i < nitems; ++i) {
         const gbt_batch_item& it = items[i];
         if (!it.volume) return fail(GBT_ERR_INVALID_ARG, "item %d has no volume", i);
-        if (it.nframes < 0 || it.first_frame < 0 || it.first_frame + it.nframes > nframes)
-            return fail(GBT_ERR_INVALID_ARG, "item %d: frames [%d, %d) outside the frame table", i, it.first_frame,
-                        it.first_frame + it.nframes);
+        if (it.nframes < 0 || it.first_frame < 0 || it.first_frame > nframes - it.nframes)   // (no sum that overflows)
+            return fail(GBT_ERR_INVALID_ARG, "item %d: frames [%d, %lld) outside the frame table", i, it.first_frame,
+                        (long long)it.first_frame + it.nframes);
     }
     return GBT_OK;
 }

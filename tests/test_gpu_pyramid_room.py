@@ -310,3 +310,16 @@ def test_images_taller_than_a_grid_of_blocks(gpu, height, with_pyramid):
     batch = BatchIntegrator(1, 1)
     assert counted(lambda: batch.integrate([vol], [[img]], [[pose]])) == (with_pyramid, with_pyramid)
     assert same(gpu, vol, bits)
+
+
+@pytest.mark.parametrize("first,count", [(2 ** 31 - 1, 1), (1, 2 ** 31 - 1), (2, 1), (0, 3), (-1, 1), (0, -1)])
+def test_item_ranges_outside_the_table_are_refused(gpu, half, first, count):
+    """Ranges whose end does not fit an int32 among them."""
+    depths, poses, cam = half
+    vol = TSDFVolume(config("frontal", (16, 16, 16), cam))
+    batch = BatchIntegrator(1, 2)
+    table = (L.Frame * 2)(*[make_frame(dev_depth(gpu, depths[0]), poses[0])] * 2)
+    items = (L.BatchItem * 1)(L.BatchItem(vol.handle.value, first, count))
+    for st in (L.lib().gbt_batch_reserve(batch._h, items, 1, table, 2),
+               L.lib().gbt_integrate_batch(batch._h, items, 1, table, 2, 128, 0, 0, None)):
+        assert st == L.GBT_ERR_INVALID_ARG and b"outside the frame table" in L.lib().gbt_last_error()
