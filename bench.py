@@ -88,11 +88,6 @@ def volume_cfg(args, cam, mode):
                             camera_width=cam.width, camera_height=cam.height, max_weight=128.0, mode=mode)
 
 
-def depth_pyramids(updates, frames, pixels):
-    """Launches of depth pyramids of a call integrating `frames` frames of `pixels` pixels (the engine's rule)."""
-    return int(updates >= (12 if frames == 1 else 8) << 20 and updates >= frames * (pixels // 2))
-
-
 class ClockSampler:
     """nvidia-smi samples (every 100 ms) of SM clock and throttle reasons
     while running.  Entering waits for nvidia-smi's first sample, so that the
@@ -889,11 +884,13 @@ def multiscene(args, torch, rank, world, local):
         step_integrate()
         step_mesh()
         torch.cuda.synchronize()
+        pyramids = L.debug_count(L.COUNT_PYRAMID_LAUNCHES)
         for fn in (step_integrate, step_mesh):
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=stream):
                 fn()
             graphs.append(g)
+        pyramids = L.debug_count(L.COUNT_PYRAMID_LAUNCHES) - pyramids   # captured: launched by every step
     g_int, g_mesh = graphs
     torch.cuda.set_stream(stream)
     for _ in range(args.warmup):
@@ -973,8 +970,7 @@ def multiscene(args, torch, rank, world, local):
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "ms_per_step": 1e3 * float(np.mean(e2e))},
         # per step: a reset per volume, the depth pyramids, the batched launches, five mesh launches per volume
-        "gpu_launches": args.steps * (6 * len(vols) + ((max(nfs) + fpl - 1) // fpl) +
-                                      depth_pyramids(updates, sum(nfs), cam.width * cam.height)),
+        "gpu_launches": args.steps * (6 * len(vols) + ((max(nfs) + fpl - 1) // fpl) + pyramids),
         "clocks": clocks.summary(),
         "autotune": {"candidates": len(table)},
     }
@@ -1262,11 +1258,13 @@ def main():
         for fn in (step_reset, step_integrate, step_mesh):   # warm the path once outside capture
             fn()
         torch.cuda.synchronize()
+        pyramids = L.debug_count(L.COUNT_PYRAMID_LAUNCHES)
         for fn in (step_reset, step_integrate, step_mesh):
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=stream):
                 fn()
             graphs.append(g)
+        pyramids = L.debug_count(L.COUNT_PYRAMID_LAUNCHES) - pyramids   # captured: launched by every step
     g_reset, g_int, g_mesh = graphs
 
     # graphs replay on the current stream: make it the stream the events go on
@@ -1439,12 +1437,9 @@ def main():
         "mesh": {"triangles_per_s": ntri / (float(np.mean(mesh_ms)) * 1e-3) if ntri else 0.0, "triangles": ntri},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "ms_per_step": float(np.mean(e2e_ms))},
-        # per step: reset, the integrate launches and their depth pyramids (one per call: the batch, or each
-        # pass), five mesh launches (bits, count, reduce, scan, emit)
-        "gpu_launches": args.steps * (1 + n_passes + 5 + (
-            depth_pyramids(nvox * nf, nf, frame_px) if path == "batched" else
-            0 if brick >= 4 else sum(depth_pyramids(nvox * k, k, frame_px)
-                                     for k in [K] * (nf // K) + [nf % K] * (nf % K > 0)))),
+        # per step: reset, the integrate launches and their depth pyramids, five mesh launches (bits, count,
+        # reduce, scan, emit)
+        "gpu_launches": args.steps * (1 + n_passes + 5 + pyramids),
         "clocks": clocks.summary(),
         "wall_s_timed": t_wall,
         "autotune": {"ns_per_update": tune["ns_per_update"], "candidates": candidates},
