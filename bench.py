@@ -1217,13 +1217,17 @@ def main():
         path, tune = ("batched", t_batched) if ms_batched < ms_single else ("single", t_single)
     K, brick, ctas = tune["frames"], tune["brick"], tune["ctas"]
     n_passes = (nf + K - 1) // K
-    # the fastest tuned candidate inside the configuration's 8-32 frames per launch
+    # the fastest tuned candidate inside the configuration's 8-32 frames per launch: the best of either
+    # path (whose tables are of different frames) on the whole sequence
     in_cfg = None
     if not args.config:
-        cands = [(ns, "batched", b_, k_, c_) for (b_, k_, c_, ns) in t_batched["table"] if k_ <= 32]
-        cands += [(ns, "single", b_, k_, c_) for (b_, k_, c_, ns) in t_single["table"] if k_ <= 32]
-        if cands:
-            in_cfg = min(cands)[1:]
+        b1, k1, c1, _ = min((r for r in t_single["table"] if r[1] <= 32), key=lambda r: r[3])
+        b2, k2, c2, _ = min((r for r in t_batched["table"] if r[1] <= 32), key=lambda r: r[3])
+        single = full_ms(lambda: (vol.reset(), vol.integrate_sequence(depths, poses, frames_per_pass=k1, brick=b1,
+                                                                      ctas_per_sm=c1)))
+        batched = full_ms(lambda: (vol.reset(), batch.integrate([vol], [depths], [poses], brick=b2, ctas_per_sm=c2,
+                                                                frames_per_launch=k2)))
+        in_cfg = ("batched", b2, k2, c2) if batched < single else ("single", b1, k1, c1)
 
     def integrate_all():
         if path == "batched":

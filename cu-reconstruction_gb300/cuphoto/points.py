@@ -99,9 +99,9 @@ class PointCloud:
         extract_points counts a slot it writes again once more, and
         set_total_number_pts the size that a cloud had before filter_depth.  The
         kernels would read and write past the points."""
-        if self.num_pts <= self.device_pts.shape[0]:
+        if self.num_pts <= self.device_pts.size(0):
             return True
-        _log("cudaPointCloud::%s() -- %d points counted, %d held" % (method, self.num_pts, self.device_pts.shape[0]))
+        _log("cudaPointCloud::%s() -- %d points counted, %d held" % (method, self.num_pts, self.device_pts.size(0)))
         return False
 
     # -- kernels ----------------------------------------------------------------
@@ -131,7 +131,7 @@ class PointCloud:
         st = L.lib().gbt_points_extract(C.byref(_k9(self.camera_matrix)), depth.data_ptr(),
                                         depth.stride(0) * (4 if f32 else 2), L.DEPTH_F32_M if f32 else L.DEPTH_U16,
                                         float(depth_scale), cptr, cpitch, W, H, C.byref(_pose7(transform)), start,
-                                        self.device_pts.data_ptr(), min(self.total_num_pts, self.device_pts.shape[0]),
+                                        self.device_pts.data_ptr(), min(self.total_num_pts, self.device_pts.size(0)),
                                         _stream_handle(stream))
         if st != L.GBT_OK:
             _log("cudaPointCloud::extract_points() -- " + L.lib().gbt_last_error().decode())
@@ -225,7 +225,7 @@ class PointCloud:
         """cudaPointCloud::add_point_cloud (cuda_point_cloud.cu:438-456)."""
         torch = _torch()
         self.device_pts = torch.cat([self.get_points(), other.get_points()]).contiguous()
-        self.num_pts = int(self.device_pts.shape[0])
+        self.num_pts = int(self.device_pts.size(0))
         self.total_num_pts = self.num_pts
         return True
 
