@@ -273,17 +273,22 @@ bool layer_runs_pay(const gbt_volume* v, int32_t n) {
     return n >= (reference ? 6 : 2);
 }
 
-// Whether depth pyramids pay for `voxel_frames` voxel-frames of work over
-// frames of `pixels` each, `frames` of them: building them is a launch of its
-// own (4.5 us) and 0.12 us for a 640x480 frame, and they save some 1.1 us per
-// million voxel-frames (0.4 of 2.8 us in 16-frame passes, 0.4 of 2.4 us for a
-// single frame), so from about five million up, unless a frame has several
-// pixels per voxel: 64^3 from one 320x240 frame takes 6.7 us without them and
-// 11.2 with, 256^3 from one 640x480 frame 39 and 27.  A single frame on its way
-// around a scene saves less: 236 x 201 x 205 takes 35.4 without and 37.2 with, so
-// for one frame the line is at twelve million.
-bool pyramids_pay(int64_t voxel_frames, int64_t frames, int64_t pixels) {
-    return voxel_frames >= (int64_t)(frames == 1 ? 12 : 8) << 20 && voxel_frames >= frames * (pixels / 2);
+// Whether depth pyramids pay for `voxel_frames` voxel-frames of work over `frames`
+// frames of up to `pixels` each.  What they save grows with the voxel-frames (some 0.2
+// us per million, more where the cameras face a surface).  They cost a launch (4.5
+// us), their frames' samples read once more (0.12 us per 640x480) and, in passes of 2
+// to 16 frames, whose lanes test a brick against one frame after the other, the
+// look-ups of those tests (0.3 us a frame).  Without / with, us, the sum over three
+// arithmetics and cameras that face the scene or circle it: 16-frame passes of
+// 640x480 at 116^3 398 / 469, 144^3 (the line) 553 / 549, 184^3 906 / 699; 8 of
+// 1280x720 at 136^3 271 / 315, 172^3 (the line) 447 / 397; 128 of 640x480 in the
+// batched kernel at 72^3 856 / 958, 88^3 (the line) 1050 / 1064, 112^3 1674 / 1348;
+// one frame at 240^3 261 / 170.  (With the line at eight million voxel-frames for any
+// number of frames, 16-frame passes of 640x480 into 92^3 took 67 to 75 us in IEEE
+// arithmetic, 47 to 60 without pyramids.)
+bool pyramids_pay(int64_t voxel_frames, int64_t frames, int64_t pixels, bool pass) {
+    const int64_t tests = pass && frames > 1 && frames <= gbt::kLaneBrickFrames ? 27 << 16 : 0;
+    return voxel_frames >= (11 << 20) + frames * (2 * pixels + tests);
 }
 
 // Tiles of room that a new volume makes: for the longest pass of frames of its
@@ -295,7 +300,7 @@ size_t first_room(const gbt_volume_cfg& c, int64_t nvox) {
     const size_t frame = gbt::pyr_tiles((int32_t)c.camera_width, (int32_t)c.camera_height);
     const size_t quarter = (size_t)nvox * 2 * sizeof(float) / 4 / sizeof(float2);
     const int64_t n = std::min((int64_t)GBT_MAX_FRAMES_PER_PASS, (int64_t)(quarter / frame));
-    return n > 0 && pyramids_pay(nvox * n, n, (int64_t)c.camera_width * c.camera_height) ? (size_t)n * frame : 0;
+    return n > 0 && pyramids_pay(nvox * n, n, (int64_t)c.camera_width * c.camera_height, true) ? (size_t)n * frame : 0;
 }
 
 // Raises d->clear, how near the camera plane boxes of voxels are tested as boxes, to
@@ -339,7 +344,7 @@ PyrPlan pass_pyramids(const gbt_volume* v, const gbt_frame* frames, int32_t n) {
         p.width = std::max(p.width, frames[i].width);
         p.height = std::max(p.height, frames[i].height);
     }
-    if (pyramids_pay(v->nvox * n, n, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
+    if (pyramids_pay(v->nvox * n, n, (int64_t)p.width * p.height, true)) p.stride = gbt::pyr_tiles(p.width, p.height);
     return p;
 }
 
@@ -1068,7 +1073,7 @@ PyrPlan batch_pyramids(const gbt_batch_item* items, int32_t nitems, const gbt_fr
     if (p.used == 0) return p;
     p.first = (uint32_t)first;
     p.frames = (uint32_t)(end - first);
-    if (pyramids_pay(work, p.used, (int64_t)p.width * p.height)) p.stride = gbt::pyr_tiles(p.width, p.height);
+    if (pyramids_pay(work, p.used, (int64_t)p.width * p.height, false)) p.stride = gbt::pyr_tiles(p.width, p.height);
     return p;
 }
 

@@ -146,6 +146,7 @@ class TSDFVolume:
         self._info = L.VolumeInfo()
         L.check(self._lib.gbt_volume_get_info(self._h, C.byref(self._info)))
         self._voxels = self._info.num_voxels
+        self._frame_pyramids = self._voxels >= self._PYRAMIDS_FROM
 
     # -- checkpoint and resume (gbt_volume_save / gbt_volume_load) -------------
     def save(self, path, stream=None):
@@ -245,7 +246,7 @@ class TSDFVolume:
             _log_error("TSDFVolume::integrate() -- depth width/height parameters are zero")
             return False
         f = make_frame(depth, camera_pose, depth_scale)
-        if self._voxels >= self._PYRAMIDS_FROM and depth.shape != self._room:
+        if self._frame_pyramids and depth.shape != self._room:
             self._lib.gbt_volume_reserve(self._h, f, 1)
             self._room = depth.shape
         st = self._lib.gbt_integrate(self._h, C.byref(f), 1, _stream_handle(stream))

@@ -170,7 +170,7 @@ gbt_status gbt_volume_transformation_voxels(gbt_volume* vol, void* stream, void*
  * for `nframes` frames at once: the frames are applied in order, in one
  * pass over the volume (distance and weight read and written once).
  * nframes may be 1..GBT_MAX_FRAMES_PER_PASS.  Asynchronous; allocates
- * nothing.  Calls of some size (from 8 M voxel-frames on) reduce each frame to a
+ * nothing.  Calls of some size (from 12 M voxel-frames on) reduce each frame to a
  * pyramid of depths first, by which parts of the volume that the frame cannot
  * update are skipped; a call for which the volume has no room for pyramids goes
  * without, with the same result in more time. */

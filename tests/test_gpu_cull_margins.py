@@ -6,14 +6,14 @@ pyramids (bricks 4-8) and the CPU oracle, bit for bit."""
 import numpy as np
 import pytest
 
-from cuphoto import TSDFVolume, TSDFVolumeConfig
+from cuphoto import TSDFVolume, TSDFVolumeConfig, _lib as L
 from cuphoto.batch import BatchIntegrator
 
 from helpers import dev_depth, oracle_run
 
 pytestmark = pytest.mark.gpu
 
-GRID, VOXEL, FRAMES = (96, 80, 72), 0.002, 16
+GRID, VOXEL, FRAMES = (152, 144, 144), 0.00125, 16
 
 
 def case(seed, offset, mode, arith):
@@ -48,15 +48,16 @@ def test_far_from_the_origin(gpu, oracle, mode, arith, offset):
     for seed in range(4):
         tc, depths, poses = case(seed, offset, mode, arith)
         dd = [dev_depth(gpu, d) for d in depths]
-        assert np.prod(GRID) * FRAMES >= 8 << 20   # with depth pyramids
 
         def bits(brick, batch=False):
             vol = TSDFVolume(tc)
+            built = L.debug_count(L.COUNT_PYRAMID_FRAMES)
             if batch:
                 BatchIntegrator(1, FRAMES).integrate([vol], [dd], [poses], brick=brick)
             else:
                 vol.integrate_frames(dd, poses, brick=brick)
             gpu.cuda.synchronize()
+            assert L.debug_count(L.COUNT_PYRAMID_FRAMES) - built == (FRAMES if brick < 4 else 0)
             return (vol.voxel_distances_data().cpu().numpy().view(np.uint32).copy(),
                     vol.voxel_weights_data().cpu().numpy().copy())
 

@@ -18,7 +18,7 @@ from test_gpu_depth_cull import config, frames, volume_bits
 
 pytestmark = pytest.mark.gpu
 
-GRID = (96, 80, 72)   # 8.8 M voxel-frames with 16 frames
+GRID = (144, 136, 140)   # 44 M voxel-frames with 16 frames
 
 
 def counted(call):
@@ -246,12 +246,11 @@ def test_creation_without_memory_for_pyramids(gpu, half, hd):
 
 
 @pytest.mark.parametrize("grid,camera,frames_with_room", [
-    ((64, 64, 64), (640, 480), 0),        # they pay from 32 frames; a quarter of the grid's 2 MB has room for 10
-    ((96, 80, 72), (640, 480), 21),       # a quarter of its bytes
     ((160, 160, 160), (640, 480), 32),
     ((160, 160, 160), (1280, 720), 32),
-    ((64, 64, 64), (1280, 720), 0),       # more than two pixels a voxel: pyramids do not pay
-    ((48, 48, 48), (640, 480), 0),        # below 8 M voxel-frames in any pass
+    ((400, 400, 400), (2560, 1920), 32),
+    ((240, 232, 236), (4096, 4096), 0),   # pyramids pay in no pass of such frames into these
+    ((96, 80, 72), (640, 480), 0),
     ((64, 64, 64), (4096, 4096), 0)])
 def test_room_at_creation_is_that_of_the_grid(gpu, grid, camera, frames_with_room):
     """How many frames of the configured camera one pass can have pyramids of,
@@ -293,11 +292,11 @@ def test_frames_that_no_item_takes_get_no_pyramid(gpu, half):
 
 @pytest.mark.parametrize("height,with_pyramid", [(65535 * 128, 1), (65535 * 128 + 1, 0)])
 def test_images_taller_than_a_grid_of_blocks(gpu, height, with_pyramid):
-    """An image of two columns and more rows than one launch's blocks cover is
+    """An image of one column and more rows than one launch's blocks cover is
     integrated without a pyramid, by single passes and by the batch."""
-    n, w = 240, 2
+    n, w = 312, 1
     tc = TSDFVolumeConfig(voxel_grid_size=(n, n, n), physical_size=(1.0, 1.0, 1.0), global_offset=(-0.5, -0.5, 0.5),
-                          focal_x=1.5, focal_y=200.0, cx=0.5, cy=150.0, camera_width=w, camera_height=300, mode="fixed")
+                          focal_x=0.75, focal_y=200.0, cx=0.0, cy=150.0, camera_width=w, camera_height=300, mode="fixed")
     img = gpu.full((height, w), 1000, dtype=gpu.int16, device="cuda")
     img[100:130] = 0
     pose = np.array([1.0, 0, 0, 0, 0, 0, 0])
