@@ -266,7 +266,9 @@ void fixed_projection(const double* pose, const gbt_volume_cfg& c, float* P) {
 // for 4, 384^3: 50.7 / 49.8 for 6, 46.4 / 44.0 for 8; IEEE arithmetic (its divides
 // leave the passes bound by instructions), 384^3: 141 / 136 for one frame, 110 /
 // 97 for 2, fixed mode 82.3 / 82.8 and 63.6 / 61.1; rows of 383 voxels, fixed: 103
-// / 89 for one, of 382, reference: 158 / 140.
+// / 89 for one, of 382, reference: 158 / 140.  (The line for the modes without
+// reference arithmetic is the fixed mode's; one IEEE compat frame, 4 % faster along z
+// at 384^3, was measured at that size alone and stays along x with it.)
 bool layer_runs_pay(const gbt_volume* v, int32_t n) {
     if (v->desc.nx % 4 != 0) return true;
     const bool reference = v->cfg.mode == GBT_MODE_COMPAT && v->cfg.arith == GBT_ARITH_REFERENCE;

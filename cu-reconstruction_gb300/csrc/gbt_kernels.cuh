@@ -1139,9 +1139,11 @@ __device__ __forceinline__ bool kinds_in_turn(const VolDesc& v, const FrameSlot*
 }
 
 // Passes of up to kLaneBrickFrames frames (LANE_BRICKS) cull with one lane
-// per brick; longer passes with one lane per frame.  The short-pass instance
-// is latency-bound: 10 resident CTAs per SM (48 registers, a few bytes of
-// spill) beat 8 at its natural 59 registers by 2-6 %.
+// per brick; longer passes with one lane per frame.  The instance with voxels
+// along x is latency-bound: in reference arithmetic, where it was measured, 10
+// resident CTAs per SM (48 registers, 8 bytes of spill) beat 8 at its natural 59
+// registers by 2-6 %.  The same bound holds the others: the IEEE compat and fixed
+// instances spill 84 to 88 bytes under it, the staged ones 60 to 160.
 // STAGE (lane-brick passes only): each warp stages the depth its voxels
 // sample in shared memory, frame by frame (gather_staged).
 // Z: see BrickLayout; the host chooses (layer_runs_pay in capi.cu).
